@@ -33,60 +33,17 @@ namespace {
 constexpr int BINS = 16;
 constexpr int MAX_LEAF = 4;
 constexpr int MAX_DEPTH = 60;
+constexpr int BUILD_THREADS = 512;  // per CTA
+constexpr int LARGE_NODE = 256;     // nodes above this are split by a CTA, the others by a warp
 constexpr unsigned FULL = 0xffffffffu;
-constexpr unsigned long long NONE_MIN = ~0ull, NONE_MAX = 0ull;
 
-// Ordering key of a float for min/max with -0 and +0 as one value (the position decides between them).
-__device__ __forceinline__ unsigned long long order_key(float v, unsigned pos, bool is_max) {
-    const float w = v == 0.0f ? 0.0f : v;
-    const unsigned u = __float_as_uint(w);
-    const unsigned k = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-    return (static_cast<unsigned long long>(k) << 32) | (is_max ? 0xffffffffu - pos : pos);
-}
-
-__device__ __forceinline__ unsigned key_pos(unsigned long long key, bool is_max) {
-    const unsigned low = static_cast<unsigned>(key);
-    return is_max ? 0xffffffffu - low : low;
-}
-
-__device__ __forceinline__ unsigned long long shfl_u64(unsigned long long v, int mask) {
-    const unsigned lo = __shfl_xor_sync(FULL, static_cast<unsigned>(v), mask);
-    const unsigned hi = __shfl_xor_sync(FULL, static_cast<unsigned>(v >> 32), mask);
-    return (static_cast<unsigned long long>(hi) << 32) | lo;
-}
-
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
-    for (int m = 16; m > 0; m >>= 1) {
-        const unsigned long long o = shfl_u64(v, m);
-        v = o < v ? o : v;
-    }
-    return v;
-}
-
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-    for (int m = 16; m > 0; m >>= 1) {
-        const unsigned long long o = shfl_u64(v, m);
-        v = o > v ? o : v;
-    }
-    return v;
-}
+// A float as an int ordered like it, -0 and +0 as one value.
+__device__ __forceinline__ int order_of(float v) { return to_ordered(v == 0.0f ? 0.0f : v); }
 
 // The host's box arithmetic (bvh::grow with std::min / std::max, bvh::surface_area).
 struct Box {
     float lo[3], hi[3];
 };
-
-__device__ __forceinline__ Box empty_box() {
-    const float inf = __int_as_float(0x7f800000);
-    return Box{{inf, inf, inf}, {-inf, -inf, -inf}};
-}
-
-__device__ __forceinline__ void grow(Box &b, const Box &o) {
-    for (int k = 0; k < 3; ++k) {
-        b.lo[k] = o.lo[k] < b.lo[k] ? o.lo[k] : b.lo[k];
-        b.hi[k] = b.hi[k] < o.hi[k] ? o.hi[k] : b.hi[k];
-    }
-}
 
 __device__ __forceinline__ float area(const Box &b) {
     const float dx = b.hi[0] - b.lo[0], dy = b.hi[1] - b.lo[1], dz = b.hi[2] - b.lo[2];
@@ -96,7 +53,7 @@ __device__ __forceinline__ float area(const Box &b) {
 
 __device__ __forceinline__ int bin_of(float c, float lo, float scale) {
     const int b = static_cast<int>((c - lo) * scale);
-    return b < BINS - 1 ? b : BINS - 1;
+    return b < 0 ? 0 : b < BINS - 1 ? b : BINS - 1;  // (never below 0 for finite vertices)
 }
 
 // Triangle boxes (the vertices' std::fmin / std::fmax in vertex order, src/mesh_build.cpp, as the host build
@@ -105,7 +62,8 @@ __device__ __forceinline__ int bin_of(float c, float lo, float scale) {
 __device__ void prepare_item(const MeshBuildArgs &a, const MeshBuildScratch &t, int i) {
     t.starts[i] = 0;
     t.top[i] = INT_MAX;
-    Box b = empty_box();
+    const float inf = __int_as_float(0x7f800000);
+    Box b{{inf, inf, inf}, {-inf, -inf, -inf}};
     for (int k = 0; k < 3; ++k) {
         const float *v = a.vertices + 3 * static_cast<size_t>(__ldg(a.indices + 3 * static_cast<size_t>(i) + k));
         for (int c = 0; c < 3; ++c) {
@@ -124,15 +82,14 @@ __device__ void prepare_item(const MeshBuildArgs &a, const MeshBuildScratch &t, 
 
 template <int WARPS>
 struct SplitSmem {
-    unsigned long long box_key[12];              // node box lo/hi (6), centroid box lo/hi (6)
-    unsigned long long bin_key[3][BINS][6];      // per axis and bin: its box lo/hi
+    int bound[12];               // node box lo/hi (6), centroid box lo/hi (6), as ordered ints
+    int bin_bound[3][BINS][6];   // per axis and bin: its box lo/hi, as ordered ints
     int bin_count[3][BINS];
-    float node[12];                              // the decoded node box and centroid box
-    float bin_box[3][BINS][6];                   // the decoded bin boxes (empty bins: +inf lo, -inf hi)
+    int zero_at[6];              // node box bounds that are zero: the first range position that holds them
     int warp_sum[WARPS];
-    int total;
-    float cbox[6];
-    int best_axis, best_bin, leaf, mid;
+    int best_axis, best_bin;
+    float best_cost;
+    int item_at[64];             // a warp's swap: the lanes of the k-th failing and the k-th passing item
 };
 
 // A barrier over the threads that split one node: the CTA, or one warp.
@@ -164,177 +121,213 @@ __device__ __forceinline__ int cta_scan(SplitSmem<WARPS> &sm, int v, bool revers
     return before + incl - v;
 }
 
-// Splits node x at this depth with a group of THREADS threads (tid: the thread's place in the group): 256 for
-// the upper depths' large nodes, one warp for the lower depths' small ones. Its children, if any, take the
-// next two places after next_first (the next depth's first node) counted by next_count.
+// The cheapest split plane over a node's bins, the axes in order, the first of equally cheap ones (src/bvh.cpp:108-125),
+// by one warp: a half warp per axis with a lane per bin, prefix and suffix boxes by shuffles (min and max in any order
+// give the host's boxes but for the sign of a zero, which no area shows).
+template <int WARPS>
+__device__ __forceinline__ void sweep_bins(SplitSmem<WARPS> &sm, const float *cb, int lane) {
+    constexpr unsigned NONE = 0xffffffffu;
+    unsigned best = NONE;
+    int best_axis = -1, best_bin = 0;
+    for (int round = 0; round < 2; ++round) {
+        const int axis = round == 0 ? lane >> 4 : 2, b = lane & 15;
+        int lo[3], hi[3], n = sm.bin_count[axis][b];
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = sm.bin_bound[axis][b][c];
+            hi[c] = sm.bin_bound[axis][b][3 + c];
+        }
+        int slo[3] = {lo[0], lo[1], lo[2]}, shi[3] = {hi[0], hi[1], hi[2]}, sn = n;
+        for (int off = 1; off < BINS; off <<= 1) {
+            const bool up = b >= off, down = b + off < BINS;
+            for (int c = 0; c < 3; ++c) {
+                const int l = __shfl_up_sync(FULL, lo[c], off, BINS), h = __shfl_up_sync(FULL, hi[c], off, BINS);
+                if (up) {
+                    lo[c] = min(lo[c], l);
+                    hi[c] = max(hi[c], h);
+                }
+                const int sl = __shfl_down_sync(FULL, slo[c], off, BINS), sh = __shfl_down_sync(FULL, shi[c], off, BINS);
+                if (down) {
+                    slo[c] = min(slo[c], sl);
+                    shi[c] = max(shi[c], sh);
+                }
+            }
+            const int k = __shfl_up_sync(FULL, n, off, BINS), q = __shfl_down_sync(FULL, sn, off, BINS);
+            if (up) n += k;
+            if (down) sn += q;
+        }
+        Box left, right;
+        for (int c = 0; c < 3; ++c) {
+            left.lo[c] = from_ordered(lo[c]);
+            left.hi[c] = from_ordered(hi[c]);
+            right.lo[c] = from_ordered(slo[c]);
+            right.hi[c] = from_ordered(shi[c]);
+        }
+        const float right_area = __shfl_down_sync(FULL, area(right), 1, BINS);
+        const int right_count = __shfl_down_sync(FULL, sn, 1, BINS);
+        unsigned key = NONE;
+        if (b < BINS - 1 && (round == 0 || lane < BINS) && cb[3 + axis] - cb[axis] > 0.0f && n != 0 && right_count != 0) {
+            const float cost = static_cast<float>(n) * area(left) + static_cast<float>(right_count) * right_area;
+            if (cost < __int_as_float(0x7f800000)) key = __float_as_uint(cost);  // never negative: ordered as an integer
+        }
+        const unsigned least = __reduce_min_sync(FULL, key);
+        if (least < best) {
+            const int at = __ffs(__ballot_sync(FULL, key == least)) - 1;
+            best = least;
+            best_axis = round == 0 ? at >> 4 : 2;
+            best_bin = at & 15;
+        }
+    }
+    if (lane == 0) {
+        sm.best_axis = best_axis;
+        sm.best_bin = best_bin;
+        sm.best_cost = best == NONE ? __int_as_float(0x7f800000) : __uint_as_float(best);
+    }
+}
+
+// Splits node x at this depth with a group of THREADS threads (tid: the thread's place in the group): a CTA for large
+// nodes, one warp for small ones. Its children, if any, take the next two places after next_first (the next depth's
+// first node) counted by next.nodes, and are listed for the next depth by size.
+// What bounds a depth is this chain of dependent steps, not work: reductions are one instruction per bound over a warp
+// (redux on ordered ints, where (value, position) pairs took ten shuffles each), bins are 32-bit shared atomics, and the
+// sweep over the bins is a scan by lanes (one thread swept the 3 x 16 bins both ways before): a depth of small nodes
+// 17 -> 6 us, a rebuild 0.66 -> 0.25 ms for 5,120 triangles and 1.45 -> 0.56 ms for 20,480 (update_mesh, B200).
 template <int THREADS>
 __device__ void split_node(const MeshBuildArgs &a, const MeshBuildScratch &t, int x, int depth, SplitSmem<THREADS / 32> &sm,
-    int tid, int next_first, int *next_count) {
+    int tid, int next_first, int *next) {
     constexpr int WARPS = THREADS / 32;
     const int lane = tid & 31;
+    const int begin = t.begin[x], end = t.end[x], count = end - begin;
+    if (tid == 0) t.depth[x] = depth;
+    for (int k = tid; k < 12; k += THREADS) sm.bound[k] = (k % 6) < 3 ? INT_MAX : INT_MIN;
+    // An empty bin is the empty box, +inf to -inf.
+    const int pos_inf = to_ordered(__int_as_float(0x7f800000)), neg_inf = to_ordered(-__int_as_float(0x7f800000));
+    for (int k = tid; k < 3 * BINS * 6; k += THREADS) (&sm.bin_bound[0][0][0])[k] = (k % 6) < 3 ? pos_inf : neg_inf;
+    for (int k = tid; k < 3 * BINS; k += THREADS) (&sm.bin_count[0][0])[k] = 0;
+    if (tid < 6) sm.zero_at[tid] = INT_MAX;
+    group_sync<WARPS>();
+
+    // The node's box and centroid box.
     {
-        const int begin = t.begin[x], end = t.end[x], count = end - begin;
-        if (tid == 0) t.depth[x] = depth;
-        for (int k = tid; k < 12; k += THREADS) sm.box_key[k] = (k % 6) < 3 ? NONE_MIN : NONE_MAX;
-        for (int k = tid; k < 3 * BINS * 6; k += THREADS)
-            (&sm.bin_key[0][0][0])[k] = (k % 6) < 3 ? NONE_MIN : NONE_MAX;
-        for (int k = tid; k < 3 * BINS; k += THREADS) (&sm.bin_count[0][0])[k] = 0;
+        int b[12];
+        for (int k = 0; k < 12; ++k) b[k] = (k % 6) < 3 ? INT_MAX : INT_MIN;
+        for (int i = begin + tid; i < end; i += THREADS) {
+            const size_t p = t.order[i];
+            for (int c = 0; c < 3; ++c) {
+                b[c] = min(b[c], order_of(t.box[6 * p + c]));
+                b[3 + c] = max(b[3 + c], order_of(t.box[6 * p + 3 + c]));
+                const int m = order_of(t.centre[3 * p + c]);
+                b[6 + c] = min(b[6 + c], m);
+                b[9 + c] = max(b[9 + c], m);
+            }
+        }
+        for (int k = 0; k < 12; ++k) {
+            const int v = (k % 6) < 3 ? __reduce_min_sync(FULL, b[k]) : __reduce_max_sync(FULL, b[k]);
+            if (lane == 0) {
+                if (WARPS == 1) sm.bound[k] = v;
+                else if ((k % 6) < 3) atomicMin(&sm.bound[k], v);
+                else atomicMax(&sm.bound[k], v);
+            }
+        }
+    }
+    group_sync<WARPS>();
+    Box box;
+    float cb[6];
+    bool zero = false;
+    for (int k = 0; k < 3; ++k) {
+        box.lo[k] = from_ordered(sm.bound[k]);
+        box.hi[k] = from_ordered(sm.bound[3 + k]);
+        cb[k] = from_ordered(sm.bound[6 + k]);
+        cb[3 + k] = from_ordered(sm.bound[9 + k]);
+        zero = zero || box.lo[k] == 0.0f || box.hi[k] == 0.0f;
+    }
+    // A box bound that is a zero has the sign of the first one in range order (the host's std::min and std::max keep
+    // the first of equal values).
+    if (zero) {
+        for (int i = begin + tid; i < end; i += THREADS) {
+            const size_t p = t.order[i];
+            for (int c = 0; c < 6; ++c)
+                if (t.box[6 * p + c] == 0.0f && (c < 3 ? box.lo[c] : box.hi[c - 3]) == 0.0f) atomicMin(&sm.zero_at[c], i);
+        }
         group_sync<WARPS>();
+        for (int c = 0; c < 6; ++c) {
+            float &v = c < 3 ? box.lo[c] : box.hi[c - 3];
+            if (v == 0.0f && sm.zero_at[c] != INT_MAX) v = t.box[6 * static_cast<size_t>(t.order[sm.zero_at[c]]) + c];
+        }
+    }
 
-        // The node's box and centroid box: per thread the first of its smallest / largest values, then the
-        // warp's and the CTA's by (value, position).
-        {
-            float best[12];
-            unsigned pos[12];
-            for (int k = 0; k < 12; ++k) {
-                best[k] = (k % 6) < 3 ? __int_as_float(0x7f800000) : -__int_as_float(0x7f800000);
-                pos[k] = 0xffffffffu;
-            }
-            for (int i = begin + tid; i < end; i += THREADS) {
-                const uint32_t p = t.order[i];
-                float v[12];
-                for (int c = 0; c < 6; ++c) v[c] = t.box[6 * static_cast<size_t>(p) + c];
-                for (int c = 0; c < 3; ++c) v[6 + c] = v[9 + c] = t.centre[3 * static_cast<size_t>(p) + c];
-                for (int k = 0; k < 12; ++k) {
-                    const bool take = (k % 6) < 3 ? v[k] < best[k] : best[k] < v[k];
-                    if (take || pos[k] == 0xffffffffu) {
-                        best[k] = v[k];
-                        pos[k] = static_cast<unsigned>(i);
-                    }
-                }
-            }
-            for (int k = 0; k < 12; ++k) {
-                const bool is_max = (k % 6) >= 3;
-                unsigned long long key = pos[k] == 0xffffffffu ? (is_max ? NONE_MAX : NONE_MIN)
-                                                                : order_key(best[k], pos[k], is_max);
-                key = is_max ? warp_max_u64(key) : warp_min_u64(key);
-                if (lane == 0) {
-                    if (is_max) atomicMax(&sm.box_key[k], key);
-                    else atomicMin(&sm.box_key[k], key);
-                }
-            }
-        }
-        group_sync<WARPS>();
-        if (tid < 12) {  // the values the keys point at, one per thread
-            const bool is_max = (tid % 6) >= 3;
-            const uint32_t p = t.order[key_pos(sm.box_key[tid], is_max)];
-            sm.node[tid] = tid < 6 ? t.box[6 * static_cast<size_t>(p) + tid] : t.centre[3 * static_cast<size_t>(p) + (tid - 6) % 3];
-        }
-        group_sync<WARPS>();
-        Box box;
-        float cb[6];
-        for (int k = 0; k < 3; ++k) {
-            box.lo[k] = sm.node[k];
-            box.hi[k] = sm.node[3 + k];
-        }
-        for (int k = 0; k < 6; ++k) cb[k] = sm.node[6 + k];
-
-        // Bins on every axis whose centroids spread (src/bvh.cpp:94-107).
-        if (count > 1) {
-            for (int i = begin + tid; i < end; i += THREADS) {
-                const uint32_t p = t.order[i];
-                for (int axis = 0; axis < 3; ++axis) {
-                    const float extent = cb[3 + axis] - cb[axis];
-                    if (!(extent > 0.0f)) continue;
-                    const float scale = static_cast<float>(BINS) / extent;
-                    const int b = bin_of(t.centre[3 * static_cast<size_t>(p) + axis], cb[axis], scale);
-                    atomicAdd(&sm.bin_count[axis][b], 1);
-                    // The shared value only moves one way, so a key that does not beat it now never will:
-                    // most keys are dropped by a plain read instead of a contended atomic.
-                    for (int c = 0; c < 6; ++c) {
-                        const bool is_max = c >= 3;
-                        const unsigned long long key = order_key(t.box[6 * static_cast<size_t>(p) + c],
-                            static_cast<unsigned>(i), is_max);
-                        unsigned long long *slot = &sm.bin_key[axis][b][c];
-                        const unsigned long long now = *reinterpret_cast<volatile unsigned long long *>(slot);
-                        if (is_max ? key > now : key < now) {
-                            if (is_max) atomicMax(slot, key);
-                            else atomicMin(slot, key);
-                        }
-                    }
+    // Bins on every axis whose centroids spread (src/bvh.cpp:94-107).
+    int best_axis = -1, best_bin = 0;
+    float best_cost = __int_as_float(0x7f800000);
+    if (count > 1) {
+        float scale[3];
+        for (int axis = 0; axis < 3; ++axis) scale[axis] = static_cast<float>(BINS) / (cb[3 + axis] - cb[axis]);
+        for (int i = begin + tid; i < end; i += THREADS) {
+            const size_t p = t.order[i];
+            int b[6];
+            for (int c = 0; c < 6; ++c) b[c] = order_of(t.box[6 * p + c]);
+            for (int axis = 0; axis < 3; ++axis) {
+                if (!(cb[3 + axis] - cb[axis] > 0.0f)) continue;
+                const int bin = bin_of(t.centre[3 * p + axis], cb[axis], scale[axis]);
+                atomicAdd(&sm.bin_count[axis][bin], 1);
+                int *slot = sm.bin_bound[axis][bin];
+                // A bound only moves one way, so a value that does not beat it now never will: most are dropped by a
+                // plain read instead of a contended atomic.
+                for (int c = 0; c < 3; ++c) {
+                    if (b[c] < *reinterpret_cast<volatile int *>(slot + c)) atomicMin(slot + c, b[c]);
+                    if (b[3 + c] > *reinterpret_cast<volatile int *>(slot + 3 + c)) atomicMax(slot + 3 + c, b[3 + c]);
                 }
             }
         }
         group_sync<WARPS>();
-        for (int e = tid; e < 3 * BINS * 6; e += THREADS) {  // the bin boxes' values, in parallel
-            const int axis = e / (BINS * 6), b = (e / 6) % BINS, c = e % 6;
-            float v = c < 3 ? __int_as_float(0x7f800000) : -__int_as_float(0x7f800000);
-            if (count > 1 && sm.bin_count[axis][b] > 0) {
-                const uint32_t p = t.order[key_pos(sm.bin_key[axis][b][c], c >= 3)];
-                v = t.box[6 * static_cast<size_t>(p) + c];
-            }
-            sm.bin_box[axis][b][c] = v;
-        }
+        if (tid < 32) sweep_bins<WARPS>(sm, cb, lane);
         group_sync<WARPS>();
-
-        // The split: the cheapest plane over the axes in order, then the leaf test (src/bvh.cpp:108-146).
-        if (tid == 0) {
-            int best_axis = -1, best_bin = 0;
-            float best_cost = __int_as_float(0x7f800000);
-            if (count > 1) {
-                for (int axis = 0; axis < 3; ++axis) {
-                    const float extent = cb[3 + axis] - cb[axis];
-                    if (!(extent > 0.0f)) continue;
-                    Box bins[BINS];
-                    for (int b = 0; b < BINS; ++b)
-                        for (int c = 0; c < 3; ++c) {
-                            bins[b].lo[c] = sm.bin_box[axis][b][c];
-                            bins[b].hi[c] = sm.bin_box[axis][b][3 + c];
-                        }
-                    float right_area[BINS - 1];
-                    int right_count[BINS - 1];
-                    Box acc = empty_box();
-                    int running = 0;
-                    for (int i = BINS - 1; i >= 1; --i) {
-                        grow(acc, bins[i]);
-                        running += sm.bin_count[axis][i];
-                        right_area[i - 1] = area(acc);
-                        right_count[i - 1] = running;
-                    }
-                    acc = empty_box();
-                    running = 0;
-                    for (int i = 0; i < BINS - 1; ++i) {
-                        grow(acc, bins[i]);
-                        running += sm.bin_count[axis][i];
-                        if (running == 0 || right_count[i] == 0) continue;
-                        const float cost = static_cast<float>(running) * area(acc) +
-                            static_cast<float>(right_count[i]) * right_area[i];
-                        if (cost < best_cost) {
-                            best_cost = cost;
-                            best_axis = axis;
-                            best_bin = i;
-                        }
-                    }
-                }
-            }
-            const float leaf_cost = static_cast<float>(count) * area(box);
-            const float split_cost = 1.0f * area(box) + best_cost;
-            const bool small = count <= MAX_LEAF;
-            sm.leaf = (count == 1 || depth >= MAX_DEPTH || (small && (best_axis < 0 || leaf_cost <= split_cost))) ? 1 : 0;
-            sm.best_axis = best_axis;
-            sm.best_bin = best_bin;
-            for (int c = 0; c < 6; ++c) sm.cbox[c] = cb[c];
-        }
+        best_axis = sm.best_axis;
+        best_bin = sm.best_bin;
+        best_cost = sm.best_cost;
+    }
+    // The leaf test (src/bvh.cpp:126-146).
+    const float leaf_cost = static_cast<float>(count) * area(box);
+    const float split_cost = 1.0f * area(box) + best_cost;
+    const bool leaf = count == 1 || depth >= MAX_DEPTH || (count <= MAX_LEAF && (best_axis < 0 || leaf_cost <= split_cost));
+    if (tid == 0)
+        for (int c = 0; c < 6; ++c) t.node_box[6 * static_cast<size_t>(x) + c] = c < 3 ? box.lo[c] : box.hi[c - 3];
+    if (leaf) {
+        if (tid == 0) t.left[x] = -1;
         group_sync<WARPS>();
-        const int leaf = sm.leaf, best_axis = sm.best_axis, best_bin = sm.best_bin;
-        if (tid < 6) t.node_box[6 * static_cast<size_t>(x) + tid] = tid < 3 ? box.lo[tid] : box.hi[tid - 3];
-        if (leaf) {
-            if (tid == 0) t.left[x] = -1;
-            group_sync<WARPS>();
-            return;
-        }
+        return;
+    }
 
-        // std::partition over the range by (bin <= best_bin): the k-th failing element from the left swaps
-        // with the k-th passing element from the right, for every k before the two runs meet.
-        int mid = begin + count / 2;
-        if (best_axis >= 0) {
-            const float lo = sm.cbox[best_axis];
-            const float scale = static_cast<float>(BINS) / (sm.cbox[3 + best_axis] - lo);
-            auto passes = [&](int i) {
-                return bin_of(t.centre[3 * static_cast<size_t>(t.order[i]) + best_axis], lo, scale) <= best_bin;
-            };
-            // Each thread takes a contiguous run of the range: it counts, the CTA scans the counts, and it
-            // writes its run's positions in order.
+    // std::partition over the range by (bin <= best_bin): the k-th failing element from the left swaps with the k-th
+    // passing element from the right, for every k before the two runs meet.
+    int mid = begin + count / 2;
+    if (best_axis >= 0) {
+        const float lo = cb[best_axis];
+        const float scale = static_cast<float>(BINS) / (cb[3 + best_axis] - lo);
+        auto passes_item = [&](uint32_t p) {
+            return bin_of(t.centre[3 * static_cast<size_t>(p) + best_axis], lo, scale) <= best_bin;
+        };
+        if (WARPS == 1 && count <= 32) {
+            // A lane per item: the ranks from ballots, the partners' lanes through shared memory.
+            const bool in = lane < count;
+            const uint32_t item = in ? t.order[begin + lane] : 0u;
+            const bool pass = in && passes_item(item);
+            const unsigned mask = __ballot_sync(FULL, pass);
+            const int passing = __popc(mask);
+            const unsigned left = passing == 32 ? FULL : (1u << passing) - 1u;
+            const unsigned fails = ~mask & left, moves = mask & ~left;  // equally many
+            const bool failing = fails >> lane & 1u, moving = moves >> lane & 1u;
+            const int k = failing ? __popc(fails & ((1u << lane) - 1u)) : __popc(moves & ~((2u << lane) - 1u));
+            if (failing) sm.item_at[k] = lane;
+            if (moving) sm.item_at[32 + k] = lane;
+            __syncwarp();
+            const int partner = failing ? sm.item_at[32 + k] : moving ? sm.item_at[k] : lane;
+            const uint32_t now = __shfl_sync(FULL, item, partner);
+            if (failing || moving) t.order[begin + lane] = now;
+            mid = begin + passing;
+        } else {
+            auto passes = [&](int i) { return passes_item(t.order[i]); };
+            // Each thread takes a contiguous run of the range: it counts, the group scans the counts, and it writes its
+            // run's positions in order.
             const int run = (count + THREADS - 1) / THREADS;
             const int r0 = begin + tid * run < end ? begin + tid * run : end;
             const int r1 = r0 + run < end ? r0 + run : end;
@@ -363,19 +356,23 @@ __device__ void split_node(const MeshBuildArgs &a, const MeshBuildScratch &t, in
                 t.order[r] = pl;
             }
             mid = meet;
-            if (mid == begin || mid == end) mid = begin + count / 2;
         }
-        group_sync<WARPS>();
-        if (tid == 0) {
-            const int c = next_first + atomicAdd(next_count, 2);
-            t.left[x] = c;
-            t.begin[c] = begin;
-            t.end[c] = mid;
-            t.begin[c + 1] = mid;
-            t.end[c + 1] = end;
-        }
-        group_sync<WARPS>();
+        if (mid == begin || mid == end) mid = begin + count / 2;
     }
+    if (tid == 0) {
+        const int c = next_first + atomicAdd(next, 2);
+        t.left[x] = c;
+        t.begin[c] = begin;
+        t.end[c] = mid;
+        t.begin[c + 1] = mid;
+        t.end[c + 1] = end;
+        for (int k = 0; k < 2; ++k) {
+            const bool large = (k == 0 ? mid - begin : end - mid) > LARGE_NODE;
+            int *list = large ? t.large : t.small;
+            list[atomicAdd(next + (large ? 1 : 2), 1)] = c + k;
+        }
+    }
+    group_sync<WARPS>();
 }
 
 // The packed tree (src/mesh_build.cpp:91-157): bvh::Node records with global indices, and the child-pair
@@ -448,15 +445,19 @@ __device__ void write_slot(const MeshBuildArgs &a, const MeshBuildScratch &t, co
     slot_hull[s].w = -1.0f;
 }
 
-// The whole build, one cooperative launch of CTAs of 256 threads; grid-wide barriers between its phases.
-__global__ void __launch_bounds__(256) build_mesh_kernel(const MeshBuildArgs a, const MeshBuildScratch t,
+// The whole build, one cooperative launch; grid-wide barriers between its phases. A depth's counts (level_count, three per
+// depth) are its nodes, and the places that its large and small nodes end at in their lists (t.large, t.small: every
+// depth's after the ones before).
+__global__ void __launch_bounds__(BUILD_THREADS, 1) build_mesh_kernel(const MeshBuildArgs a, const MeshBuildScratch t,
     const int *slot_mesh, int slots, int mesh, int2 *slot_root, float *slot_bounds, float4 *slot_hull) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    __shared__ SplitSmem<8> cta_smem;
-    __shared__ SplitSmem<1> warp_smem[8];
-    __shared__ int prefix_warp[8];
-    __shared__ int prefix_carry;
+    constexpr int WARPS = BUILD_THREADS / 32;
+    __shared__ union {
+        SplitSmem<WARPS> cta;
+        SplitSmem<1> warp[WARPS];
+    } smem;
+    __shared__ int prefix_warp[WARPS];
     const long long rank = grid.thread_rank(), size = grid.size();
     const int T = a.triangles;
     const long long cap = 2LL * T - 1;
@@ -466,7 +467,7 @@ __global__ void __launch_bounds__(256) build_mesh_kernel(const MeshBuildArgs a, 
     for (long long k = rank; k < 2 * cap; k += size) a.blas[2LL * a.node_base + k] = zero;
     for (long long k = rank; k < 4 * cap; k += size) a.pairs[4LL * a.node_base + k] = zero;
     for (long long i = rank; i < T; i += size) prepare_item(a, t, static_cast<int>(i));
-    for (long long d = rank; d <= MESH_LEVELS; d += size) t.level_count[d] = 0;
+    for (long long d = rank; d < 3 * (MESH_LEVELS + 1); d += size) t.level_count[d] = 0;
     if (rank == 0) {
         t.begin[0] = 0;
         t.end[0] = T;
@@ -474,22 +475,28 @@ __global__ void __launch_bounds__(256) build_mesh_kernel(const MeshBuildArgs a, 
     }
     grid.sync();
 
-    // Depth after depth: the splits of depth d append depth d + 1's nodes after depth d's last.
-    int first = 0, last = 1;
+    // Depth after depth: the splits of depth d append depth d + 1's nodes after depth d's last, and list them by size.
+    // A depth's lists start where the one before ended: list positions are counted from there.
+    int first = 0, last = 1, large0 = 0, large1 = T > LARGE_NODE ? 1 : 0, small0 = 0, small1 = 1 - large1;
     for (int depth = 0; depth < MESH_LEVELS && first < last; ++depth) {
-        int *next_count = t.level_count + depth + 1;
-        if ((static_cast<long long>(T) >> depth) > 512) {
-            for (int x = first + blockIdx.x; x < last; x += gridDim.x)
-                split_node<256>(a, t, x, depth, cta_smem, threadIdx.x, last, next_count);
-        } else {
-            const int w = threadIdx.x >> 5;
-            for (int x = first + blockIdx.x * 8 + w; x < last; x += gridDim.x * 8)
-                split_node<32>(a, t, x, depth, warp_smem[w], threadIdx.x & 31, last, next_count);
-        }
+        int *next = t.level_count + 3 * (depth + 1);
+        MeshBuildScratch u = t;
+        u.large = t.large + large1;
+        u.small = t.small + small1;
+        for (int k = large0 + blockIdx.x; k < large1; k += gridDim.x)
+            split_node<BUILD_THREADS>(a, u, depth == 0 ? 0 : t.large[k], depth, smem.cta, threadIdx.x, last, next);
+        __syncthreads();
+        const int w = threadIdx.x >> 5;
+        // Small nodes over the CTAs first, then over a CTA's warps.
+        for (int k = small0 + blockIdx.x + gridDim.x * w; k < small1; k += gridDim.x * WARPS)
+            split_node<32>(a, u, depth == 0 ? 0 : t.small[k], depth, smem.warp[w], threadIdx.x & 31, last, next);
         grid.sync();
-        const int next = last + __ldcg(next_count);
         first = last;
-        last = next;
+        last += __ldcg(next);
+        large0 = large1;
+        large1 += __ldcg(next + 1);
+        small0 = small1;
+        small1 += __ldcg(next + 2);
     }
     const int nodes = last;
 
@@ -503,24 +510,32 @@ __global__ void __launch_bounds__(256) build_mesh_kernel(const MeshBuildArgs a, 
         }
     grid.sync();
     if (blockIdx.x == 0) {
+        constexpr int RUN = 8;  // consecutive positions per thread
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        if (threadIdx.x == 0) prefix_carry = 0;
-        __syncthreads();
-        for (int base = 0; base < T; base += 256) {
-            const int i = base + threadIdx.x;
-            const int v = i < T ? __ldcg(t.starts + i) : 0;
-            int incl = v;
+        int carry = 0;
+        for (int base = 0; base < T; base += BUILD_THREADS * RUN) {
+            const int i0 = base + threadIdx.x * RUN;
+            int v[RUN], sum = 0;
+            for (int k = 0; k < RUN; ++k) {
+                v[k] = i0 + k < T ? __ldcg(t.starts + i0 + k) : 0;
+                sum += v[k];
+            }
+            int incl = sum;
             for (int o = 1; o < 32; o <<= 1) {
                 const int u = __shfl_up_sync(FULL, incl, o);
                 if (lane >= o) incl += u;
             }
             if (lane == 31) prefix_warp[warp] = incl;
             __syncthreads();
-            int before = prefix_carry;
-            for (int k = 0; k < warp; ++k) before += prefix_warp[k];
-            if (i < T) t.prefix[i] = before + incl - v;
-            __syncthreads();
-            if (threadIdx.x == 255) prefix_carry = before + incl;
+            int at = carry + incl - sum;
+            for (int k = 0; k < WARPS; ++k) {
+                if (k < warp) at += prefix_warp[k];
+                carry += prefix_warp[k];
+            }
+            for (int k = 0; k < RUN; ++k) {
+                if (i0 + k < T) t.prefix[i0 + k] = at;
+                at += v[k];
+            }
             __syncthreads();
         }
     }
@@ -550,7 +565,7 @@ cudaError_t launch_mesh_build(const MeshBuildArgs &a, const MeshBuildScratch &t,
     int device = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, build_mesh_kernel, 256, 0);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, build_mesh_kernel, BUILD_THREADS, 0);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     // Every CTA resident at once (the barriers need it); no more CTAs than about one per 8 triangles.
@@ -561,7 +576,7 @@ cudaError_t launch_mesh_build(const MeshBuildArgs &a, const MeshBuildScratch &t,
     void *args[] = {const_cast<MeshBuildArgs *>(&a), const_cast<MeshBuildScratch *>(&t), &slot_mesh, &slots, &mesh,
         &slot_root, &slot_bounds, &slot_hull};
     return cudaLaunchCooperativeKernel(reinterpret_cast<void *>(build_mesh_kernel), dim3(static_cast<unsigned>(blocks)),
-        dim3(256), args, 0, stream);
+        dim3(BUILD_THREADS), args, 0, stream);
 }
 
 }  // namespace ngb

@@ -158,9 +158,13 @@ cudaError_t launch_rays_persistent(const SceneParams &s, const RayArgs &r, int *
 // Ray queries as warp packets over each world's tree: 32 consecutive rays of a world per warp (see tiles.cu).
 cudaError_t launch_rays_packets(const SceneParams &s, const RayArgs &r, int *counter, cudaStream_t stream);
 
-// The tile render: the persistent kernel's cases, for worlds of at most TILE_MAX_INSTANCES instances (see
-// tiles.cu). Of the tuning, threads and registers are read: 128/48, 128/56, 128/64, 128/80 or 256/64.
-constexpr int TILE_MAX_INSTANCES = 256;
+// The tile render (see tiles.cu). Of the tuning, threads and registers are read: 128/48, 128/56, 128/64, 128/80 or
+// 256/64. counters: tile_counters(a, lights) zeroed counters, one for each launch that takes tiles from a queue.
+constexpr int TILE_MAX_INSTANCES = 256;  // the largest world rendered from candidate lists
+inline bool one_pass(const RenderArgs &a, int lights) { return a.spp == 1 && lights <= 1 && !a.reflective; }
+inline size_t tile_counters(const RenderArgs &a, int lights) {
+    return !a.rgb ? 1 : one_pass(a, lights) ? 2 : static_cast<size_t>(a.spp) * (2 + lights);
+}
 // after_camera / after_shade (may be null) are recorded on the stream after the camera and shade kernels.
 cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, int *counter, const PersistentTuning &t,
     cudaStream_t stream, cudaEvent_t after_camera, cudaEvent_t after_shade);
@@ -218,7 +222,9 @@ struct MeshBuildScratch {
     int *depth;                 // per node
     int *index;                 // per node: its index in the mesh's tree
     int *counter;               // out: the tree's node count
-    int *level_count;           // per depth (MESH_LEVELS + 1): the nodes its parents' splits appended
+    int *level_count;           // per depth (MESH_LEVELS + 1), 3: the nodes its parents' splits appended, and how many of
+                                // them are large and small
+    int *large, *small;         // the large and the small nodes, depth after depth (cap each)
     int *starts, *top, *prefix; // per order position: internal nodes starting there, the least depth of those,
                                 // and the internal nodes starting before it
 };

@@ -192,7 +192,7 @@ struct Renderer {
     DevBuf<float> mb_box, mb_centre, mb_node_box;
     DevBuf<uint32_t> mb_order;
     DevBuf<int> mb_lpos, mb_rpos, mb_begin, mb_end, mb_left, mb_depth, mb_index, mb_counter, mb_starts, mb_top, mb_prefix;
-    DevBuf<int> mb_level_count;
+    DevBuf<int> mb_level_count, mb_large, mb_small;
     int *host_count = nullptr;  // pinned: a level's node count read back during a mesh rebuild
     // Staging for host inputs and the renderer's own outputs.
     DevBuf<float> cameras, ray_origins, ray_directions;
@@ -571,7 +571,7 @@ void Renderer::teardown() {
     mb_box.release(), mb_centre.release(), mb_node_box.release(), mb_order.release(), mb_lpos.release();
     mb_rpos.release(), mb_begin.release(), mb_end.release(), mb_left.release(), mb_depth.release();
     mb_index.release(), mb_counter.release(), mb_starts.release(), mb_top.release(), mb_prefix.release();
-    mb_level_count.release();
+    mb_level_count.release(), mb_large.release(), mb_small.release();
     blas_pairs.release(), tlas_pairs.release(), slot_root.release(), work_counter.release();
     large_aabb.release(), large_bounds.release(), large_ids_a.release(), large_ids_b.release();
     large_keys_a.release(), large_keys_b.release(), large_counts.release();
@@ -859,7 +859,9 @@ void Renderer::update_mesh(int mesh, const float *vertices, const float *normals
     t.depth = mb_depth.ensure(cap);
     t.index = mb_index.ensure(cap);
     t.counter = mb_counter.ensure(1);
-    t.level_count = mb_level_count.ensure(MESH_LEVELS + 1);
+    t.level_count = mb_level_count.ensure(3 * (MESH_LEVELS + 1));
+    t.large = mb_large.ensure(cap);
+    t.small = mb_small.ensure(cap);
     t.starts = mb_starts.ensure(T);
     t.top = mb_top.ensure(T);
     t.prefix = mb_prefix.ensure(T);
