@@ -111,6 +111,15 @@ struct RenderArgs {
     int *view_order;
     float *view_bound;
     int order_stride;
+    // Pictures of several samples, lights or mirror bounces on the tile kernels (see tiles.cu, sample passes).
+    int reflective;                // some material bounces light
+    int sample;                    // the sample this pass traces
+    const uint32_t *rng_in;        // per pixel: the random stream where the sample starts it, or null (the first sample)
+    uint32_t *rng_out;             // per pixel: where the sample leaves it
+    float4 *sample_sum;            // per pixel: the sum of the samples so far
+    uint8_t *visible;              // per pixel: bit i set while light i is not found blocked
+    int light;                     // the light whose shadow rays this pass traces
+    int *bounces;                  // how many pixels' paths go on from a mirror
 };
 
 // The running average of a single-view renderer's pictures (render_pixel, src/render_core.h:288-301): per pixel
@@ -166,7 +175,7 @@ inline size_t tile_counters(const RenderArgs &a, int lights) {
     return !a.rgb ? 1 : one_pass(a, lights) ? 2 : static_cast<size_t>(a.spp) * (2 + lights);
 }
 // after_camera / after_shade (may be null) are recorded on the stream after the camera and shade kernels.
-cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, int *counter, const PersistentTuning &t,
+cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, unsigned long long *counters, const PersistentTuning &t,
     cudaStream_t stream, cudaEvent_t after_camera, cudaEvent_t after_shade);
 
 // The adjoint of the depth and normal images (see adjoint.cu). Every pointer is device memory; grad_normal

@@ -156,6 +156,9 @@ struct Renderer {
     DevBuf<float4> camera_basis;              // the persistent and tile renders' per-view cameras
     DevBuf<float4> pic_hit, shadow_o, shadow_d;  // the tile render's per-pixel hand-over between its kernels
     DevBuf<int> pic_code, shadow_self;
+    DevBuf<uint32_t> sample_rng;              // between the samples of a picture (tiles.cu, sample passes)
+    DevBuf<float4> sample_sum;
+    DevBuf<uint8_t> sample_visible;
     DevBuf<int> view_order;                   // the tile render's per-view candidate order, and its bounds
     DevBuf<float> view_bound;
     DevBuf<float> srgb_table;                 // 256 sRGB byte thresholds
@@ -264,6 +267,7 @@ struct Renderer {
     void put_lights(const ngb_light *lights, int count);
     void cast_rays(const float *o, const float *d, int rays_per_world, float max_distance, int memory, ngb_ray_hits *out,
         float *distance, float *normal, int32_t *ids);
+    bool pass_scratch(const RenderArgs &a, int views, bool single);
     int rows() const { return band_rows > 0 ? band_rows : height; }
     size_t pixels() const {
         return uneven ? static_cast<size_t>(total_pixels) : static_cast<size_t>(worlds) * cpw * rows() * width;
@@ -575,6 +579,7 @@ void Renderer::teardown() {
     blas_pairs.release(), tlas_pairs.release(), slot_root.release(), work_counter.release();
     large_aabb.release(), large_bounds.release(), large_ids_a.release(), large_ids_b.release();
     large_keys_a.release(), large_keys_b.release(), large_counts.release();
+    sample_rng.release(), sample_sum.release(), sample_visible.release();
     pic_hit.release(), shadow_o.release(), shadow_d.release(), pic_code.release(), shadow_self.release();
     view_order.release(), view_bound.release();
     leaf_of.release(), slot_hull.release(), slot_sphere.release();
@@ -946,6 +951,32 @@ void Renderer::check_view(const ngb_camera *c, int frame, int spp) {
     require(all_finite(v, 14), "camera has a NaN or infinite value (is its target on the view axis, or up parallel to it?)");
 }
 
+// The tile kernels' scratch for a render that the per-pixel kernel could do too: false where it cannot be had (no
+// memory left, not allocated yet when a capture forbids it, or more pixels than the passes' lists can name).
+bool Renderer::pass_scratch(const RenderArgs &a, int views, bool single) {
+    const size_t px = pixels(), nv = static_cast<size_t>(views);
+    if (px > static_cast<size_t>(INT32_MAX)) return false;
+    const bool fixed = capturing();
+    auto have = [&](auto &buf, size_t count) {
+        if (fixed) return buf.n >= count;
+        buf.ensure(count);
+        return true;
+    };
+    try {
+        bool ok = have(camera_basis, 3 * nv) && have(work_counter, tile_counters(a, params.light_count));
+        if (per_world > 0 && per_world <= TILE_MAX_INSTANCES)
+            ok = ok && have(view_order, nv * per_world) && have(view_bound, nv * per_world);
+        if (a.rgb)
+            ok = ok && have(pic_hit, px) && have(pic_code, px) && have(shadow_o, px) && have(shadow_d, px) &&
+                have(shadow_self, px);
+        if (!single) ok = ok && have(sample_rng, px) && have(sample_sum, px) && have(sample_visible, px);
+        return ok;
+    } catch (const CudaFailure &) {
+        cudaGetLastError();
+        return false;
+    }
+}
+
 void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, int frame, int memory, uint8_t *rgb,
     float *depth, float *normal, int32_t *ids, const ngb_camera *view) {
     Range range(view ? "ngb render_view" : "ngb render");
@@ -999,12 +1030,18 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         }
     }
     a.error_flag = error_flag.p;
-    // The persistent and tile kernels cover one sample per pixel, at most one light and no bounces; everything
-    // else takes the per-pixel kernel, which runs trace in full. Automatic: the tile kernels (candidate lists
-    // for worlds of at most TILE_MAX_INSTANCES instances, a packet walk of the world tree above).
+    // Automatic: the tile kernels (candidate lists for worlds of at most TILE_MAX_INSTANCES instances, a packet walk of
+    // the world tree above), in one pass for one sample per pixel, at most one light and no mirrors, else in
+    // several. The persistent kernel covers only the first of these; the per-pixel kernel runs trace in full.
     const bool persistent_ok = spp == 1 && params.light_count <= 1 && !reflective;
     // A view render's picture is a running average of radiance, which the tile and per-pixel kernels hand over.
-    const bool tiles = persistent_ok && (uneven || kernel_choice == 3 || kernel_choice == 0 || (view && kernel_choice == 2));
+    a.reflective = reflective ? 1 : 0;
+    const bool single = (outputs & NGB_OUTPUT_RGB) == 0 || one_pass(a, params.light_count);
+    bool tiles = uneven ? persistent_ok
+        : (kernel_choice == 3 || kernel_choice == 0 || (view && kernel_choice == 2 && persistent_ok));
+    // The per-pixel kernel needs no scratch: pictures that the tile kernels take several passes for go to it where the
+    // passes' scratch cannot be had.
+    if (tiles && !persistent_ok) tiles = pass_scratch(a, views, single);
     const bool persistent = !view && !tiles && persistent_ok && (kernel_choice == 0 || kernel_choice == 2);
     if (view && a.rgb) {
         a.radiance = view_radiance.ensure(pixels());
@@ -1041,9 +1078,14 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
             a.shadow_d = shadow_d.ensure(pixels());
             a.shadow_self = shadow_self.ensure(pixels());
         }
-        CK(launch_render_tiles(params, a, reinterpret_cast<int *>(work_counter.p), tile_tuning, stream,
+        if (!single) {
+            a.rng_out = sample_rng.ensure(pixels());
+            a.sample_sum = sample_sum.ensure(pixels());
+            a.visible = sample_visible.ensure(pixels());
+        }
+        CK(launch_render_tiles(params, a, work_counter.ensure(tile_counters(a, params.light_count)), tile_tuning, stream,
             timed ? ev_stage[0] : nullptr, timed ? ev_stage[1] : nullptr));
-        stages = 3;
+        stages = single ? 3 : 1;
     } else if (persistent) {
         a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
         CK(launch_render_persistent(params, a, reinterpret_cast<int *>(work_counter.p), tuning, stream));

@@ -302,6 +302,94 @@ __device__ __forceinline__ void packet_walk(const SceneParams &s, WarpSmem<0> &s
     }
 }
 
+// A world's tree walked by each lane for itself, for rays that share no more than their kernel (bounces off mirrors): the
+// reference's walk, order and all (traverse<true>, src/mesh_dev.h:113-159), from child-pair records. A lane walks down
+// to the next instance its ray enters, and the warp's lanes then walk the instances they stand at together, each its
+// own (one walk site, inlined).
+// ANY: true at the first hit closer than tmax (hit_inst set). skip: an instance the lane leaves out (-1: none).
+template <bool ANY>
+__device__ __forceinline__ void lane_walk(const SceneParams &s, int world, float3 o, float3 d, float &tmax,
+    int &hit_inst, int &hit_tri, float &hu, float &hv, int skip, int max_steps, int *err) {
+    const int root = s.instance_count > 0 ? __ldg(s.roots + world) : -1;
+    if (root < 0) return;
+    const float3 inv = safe_inverse(d);
+    int4 st[TLAS_STACK];  // (reference, count, entry distance) per pushed node, stored and loaded whole
+    int ref = root, count = 0, sp = 0;
+    const float4 lo = __ldg(s.tlas + 2 * root), hi = __ldg(s.tlas + 2 * root + 1);
+    if (box_entry(lo, hi, o, inv, tmax) >= NO_HIT) return;
+    if (root >= s.tlas_internal) {  // a world of one instance: its leaf is the root
+        ref = ~__float_as_int(lo.w);
+        count = -1;
+    }
+    const int max_nodes = 2 * s.instance_count + 2;
+    int steps = 0;
+    for (;;) {
+        bool out = false;
+        while (count == 0) {
+            if (++steps > max_nodes) {  // a correct walk visits each node once; only a malformed tree gets here
+                *err = 2;
+                return;
+            }
+            const float4 *q = s.tlas_pairs + 4 * static_cast<long long>(ref);
+            const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
+            const float dl = box_entry(make_float4(q0.x, q0.y, q0.z, 0.0f), make_float4(q0.w, q1.x, q1.y, 0.0f), o, inv,
+                tmax);
+            const float dr = box_entry(make_float4(q1.z, q1.w, q2.x, 0.0f), make_float4(q2.y, q2.z, q2.w, 0.0f), o, inv,
+                tmax);
+            if (dl < NO_HIT || dr < NO_HIT) {
+                const bool left_first = dl <= dr;
+                const float far_t = left_first ? dr : dl;
+                if (far_t < NO_HIT) {
+                    if (sp >= TLAS_STACK) {
+                        *err = 1;
+                        return;
+                    }
+                    st[sp++] = make_int4(__float_as_int(left_first ? q3.z : q3.x), __float_as_int(left_first ? q3.w : q3.y),
+                        __float_as_int(far_t), 0);
+                }
+                ref = __float_as_int(left_first ? q3.x : q3.z);
+                count = __float_as_int(left_first ? q3.y : q3.w);
+            } else {
+                int4 e = make_int4(0, 0, 0, 0);
+                while (sp > 0) {
+                    e = st[sp - 1];
+                    if (__int_as_float(e.z) < tmax) break;
+                    --sp;
+                }
+                if (sp == 0) {
+                    out = true;
+                    break;
+                }
+                --sp;
+                ref = e.x;
+                count = e.y;
+            }
+        }
+        if (out) return;
+        if (ANY) {
+            float tm = tmax;
+            if (ref != skip && instance_walk_body<true>(s.inst, s.slot_bounds, s.slot_root, s.blas_pairs, s.tris,
+                                   s.slot_sphere, ref, o, d, tm, hit_tri, hu, hv, max_steps, err)) {
+                hit_inst = ref;
+                return;
+            }
+        } else if (instance_walk_body<false>(s.inst, s.slot_bounds, s.slot_root, s.blas_pairs, s.tris, s.slot_sphere, ref,
+                       o, d, tmax, hit_tri, hu, hv, max_steps, err)) {
+            hit_inst = ref;
+        }
+        int4 e = make_int4(0, 0, 0, 0);
+        while (sp > 0) {
+            e = st[sp - 1];
+            if (__int_as_float(e.z) < tmax) break;
+            --sp;
+        }
+        if (sp == 0) return;
+        --sp;
+        ref = e.x;
+        count = e.y;
+    }
+}
+
 // Spheres and the floor before the meshes, the meshes with the closest of those as their limit
 // (scene_intersect, src/render_core.h:78-112).
 __device__ __forceinline__ float spheres_and_floor(const SceneParams &s, float3 o, float3 d, int &best_sphere,
@@ -504,11 +592,14 @@ __device__ __forceinline__ long long fetch_tiles(int *counter, int lane, int fet
     return __shfl_sync(FULL, first, 0);
 }
 
-// The picture ray of pixel (x, y): its jitter draws from the pixel's random stream, which is left where the
-// light sample continues it (sample_pixel, src/render_core.h:248-258).
-__device__ __forceinline__ float3 picture_ray(const RenderArgs &a, int x, int y, int width, int height, float aspect,
-    float3 right, float3 up, float3 fwd, uint32_t &rng) {
-    rng = pcg_hash(static_cast<uint32_t>(y * width + x) ^ pcg_hash(static_cast<uint32_t>(a.frame) + 1u));
+// The picture ray of pixel (x, y), index pix: its jitter draws from the pixel's random stream, which is left where the
+// light sample continues it (sample_pixel, src/render_core.h:248-258). LATER: not the pixel's first sample, whose stream
+// starts where the one before left it.
+template <bool LATER>
+__device__ __forceinline__ float3 picture_ray(const RenderArgs &a, int x, int y, long long pix, int width, int height,
+    float aspect, float3 right, float3 up, float3 fwd, uint32_t &rng) {
+    rng = LATER ? a.rng_in[pix]
+                : pcg_hash(static_cast<uint32_t>(y * width + x) ^ pcg_hash(static_cast<uint32_t>(a.frame) + 1u));
     const float jx = rand_float(rng);
     const float jy = rand_float(rng);
     return camera_dir(right, up, fwd, static_cast<float>(x) + jx, static_cast<float>(y) + jy, static_cast<float>(width),
@@ -519,10 +610,10 @@ __device__ __forceinline__ float3 picture_ray(const RenderArgs &a, int x, int y,
 // (instance >= 0, else -1 nothing, -2 the floor, -3 - i sphere i).
 constexpr int CODE_NONE = -1, CODE_FLOOR = -2, CODE_SPHERE = -3;
 
-// Camera kernel. THREADS per CTA and MIN_BLOCKS resident CTAs per SM set the register budget. Per tile: the
+// Camera kernel (LATER: the picture rays of a sample after a pixel's first). THREADS per CTA and MIN_BLOCKS resident CTAs per SM set the register budget. Per tile: the
 // candidates, then the centre rays (depth, normals, IDs written here) and the picture rays (their closest
 // hits written for the shade kernel).
-template <int THREADS, int MIN_BLOCKS, int CAP, bool PAIRED>
+template <int THREADS, int MIN_BLOCKS, int CAP, bool PAIRED, bool LATER = false>
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) camera_tiles_kernel(const __grid_constant__ SceneParams s,
     const RenderArgs a, int *counter, long long tiles, int tiles_x, int tiles_per_view, int fetch) {
     __shared__ WarpSmem<CAP> warp_smem[THREADS / 32];
@@ -621,7 +712,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) camera_tiles_kernel(const
                         fs, asp);
                 } else {
                     uint32_t rng;
-                    d = picture_ray(a, T.x, T.y, T.width, T.height, asp, right, up, fwd, rng);
+                    d = picture_ray<LATER>(a, T.x, T.y, T.pix, T.width, T.height, asp, right, up, fwd, rng);
                 }
                 int best_sphere;
                 bool hit_floor;
@@ -719,7 +810,7 @@ __device__ __forceinline__ bool shadow_misses_own_mesh(const SceneParams &s, int
 // RADIANCE: a single-view render's kernel (a.radiance set), keeping each pixel's radiance for its running average;
 // otherwise the batch's, writing bytes.
 template <bool RADIANCE>
-__global__ void __launch_bounds__(256) shade_kernel(const __grid_constant__ SceneParams s, const RenderArgs a,
+__global__ void __launch_bounds__(128, 8) shade_kernel(const __grid_constant__ SceneParams s, const RenderArgs a,
     long long pixels) {
     const long long per_view = static_cast<long long>(a.width) * a.rows;
     const float3 zero = mk3(0.0f, 0.0f, 0.0f);
@@ -746,7 +837,7 @@ __global__ void __launch_bounds__(256) shade_kernel(const __grid_constant__ Scen
         const float3 eye = mk3(c0.x, c0.y, c0.z), right = mk3(c0.w, c1.x, c1.y);
         const float3 up = mk3(c1.z, c1.w, c2.x), fwd = mk3(c2.y, c2.z, c2.w);
         uint32_t rng;
-        const float3 d = picture_ray(a, x, y, width, height, aspect, right, up, fwd, rng);
+        const float3 d = picture_ray<false>(a, x, y, p, width, height, aspect, right, up, fwd, rng);
         const int code = a.pic_code[p];
         const float4 h = a.pic_hit[p];
         float3 radiance, shadowed = zero;
@@ -855,7 +946,8 @@ __global__ void __launch_bounds__(256) shade_kernel(const __grid_constant__ Scen
 // Separating axes: x, y and z, the direction away from the light, and four axes tilted from the sideways
 // directions towards the light by the light sphere's angular radius, which hug the hull's sides. Each support
 // is taken over the segments' own end points, so any axis is a valid test; these make it a tight one.
-template <int THREADS, int MIN_BLOCKS, int CAP>
+// BITS: of a picture's sample passes (the answers are bits of visible, the light is a.light).
+template <int THREADS, int MIN_BLOCKS, int CAP, bool BITS>
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_tiles_kernel(const __grid_constant__ SceneParams s,
     const RenderArgs a, int *counter, long long tiles, int tiles_x, int tiles_per_view, int fetch) {
     __shared__ int warp_cand[THREADS / 32][CAP];
@@ -863,7 +955,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_tiles_kernel(const
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     const int max_steps = s.blas_node_count + 2;
-    const DevLight &lt = s.lights[0];
+    const DevLight &lt = s.lights[BITS ? a.light : 0];
     const float INF = __int_as_float(0x7f800000);
     for (;;) {
         const long long first = fetch_tiles(counter, lane, fetch);
@@ -964,7 +1056,9 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_tiles_kernel(const
                         s.slot_sphere, id, so, sd, tm, ht, hu, hv, max_steps, a.error_flag);
                 }
             }
-            if (pending && a.radiance) {
+            if (BITS) {
+                if (blocked) a.visible[T.pix] &= static_cast<uint8_t>(~(1u << a.light));
+            } else if (pending && a.radiance) {
                 if (blocked) a.radiance[T.pix] = a.pic_hit[T.pix];
             } else if (pending) {
                 put_rgb(a.rgb, T.pix, blocked ? a.pic_code[T.pix] : __float_as_int(d4.w));
@@ -977,7 +1071,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_tiles_kernel(const
 // pending shadow rays (those the shade kernel left) walk the world's tree together, a lane stopping at its first
 // hit (packet_walk<true>); a lane leaves out its own mesh where the shade kernel found the ray cannot meet it.
 // Neighbouring pixels' rays leave nearby points for the same light, so they enter nearly the same nodes.
-template <int THREADS, int MIN_BLOCKS>
+template <int THREADS, int MIN_BLOCKS, bool BITS>
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_packets_kernel(const __grid_constant__ SceneParams s,
     const RenderArgs a, int *counter, long long tiles, int tiles_x, int tiles_per_view, int fetch) {
     __shared__ WarpSmem<0> warp_smem[THREADS / 32];
@@ -1006,7 +1100,9 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_packets_kernel(con
             packet_walk<true>(s, sm, lane, T.world, pending, mk3(o4.x, o4.y, o4.z), mk3(d4.x, d4.y, d4.z), tmax,
                 hit_inst, hit_tri, hu, hv, skip, max_steps, a.error_flag);
             const bool blocked = hit_inst >= 0;
-            if (pending && a.radiance) {
+            if (BITS) {
+                if (blocked) a.visible[T.pix] &= static_cast<uint8_t>(~(1u << a.light));
+            } else if (pending && a.radiance) {
                 if (blocked) a.radiance[T.pix] = a.pic_hit[T.pix];
             } else if (pending) {
                 put_rgb(a.rgb, T.pix, blocked ? a.pic_code[T.pix] : __float_as_int(d4.w));
@@ -1066,27 +1162,305 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) ray_packets_kernel(const 
 }
 
 template <class Kernel>
-cudaError_t launch_tiles(Kernel kernel, int threads, const SceneParams &s, const RenderArgs &a, int *counter,
-    long long tiles, int tiles_x, int tiles_per_view, int fetch, cudaStream_t stream) {
+cudaError_t launch_tiles(Kernel kernel, int threads, const SceneParams &s, const RenderArgs &a,
+    unsigned long long *counter, long long tiles, int tiles_x, int tiles_per_view, int fetch, cudaStream_t stream) {
     int device = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
+// ------------------------------------------------------------------------------------------------------
+// Sample passes: pictures of several samples per pixel, several lights, or mirrors, on the same tile kernels. Per sample:
+// the camera kernel (its picture rays only after the first sample), then for each light a light_kernel that leaves
+// the light's shadow rays and the shadow kernel that answers them (a bit per pixel and light), then finish_kernel,
+// which lights each hit with the lights found visible and adds the sample to the pixel's sum; where the hit is a mirror
+// it lists the path for bounce_kernel, which follows the paths that go on, bounce by bounce. The
+// arithmetic and its order are trace's (trace_common.cuh; src/render_core.h:202-283), so the sums are the per-pixel
+// kernel's bit for bit. The pixel's random stream passes from sample to sample through memory (rng_out), since how far
+// a sample draws depends on what it hits.
+// Why: the per-pixel kernel walks each of these rays alone (a pixel's samples, lights and bounces one after the
+// other in one thread, every warp waiting for its slowest lane at each); the tile kernels walk neighbouring rays
+// together from culled lists. 96 worlds of 20 instances at 96 x 96, four samples, two lights, a fifth of the instances
+// mirrors: 7.0 ms on the per-pixel kernel, 2.7 ms here (camera 0.6, lights and finishing 0.4, shadows 0.75, bounces 0.9).
+
+// Pixel p of views of one size, its view's camera and its picture ray, with the random stream just past the jitter.
+struct PixelRay {
+    int world;
+    float3 eye, d;
+    uint32_t rng;
+};
+__device__ __forceinline__ PixelRay pixel_ray(const RenderArgs &a, long long p) {
+    int rem;
+    const int view = split_index(p, a.width * a.rows, rem);
+    const int y = a.row_first + rem / a.width, x = rem % a.width;
+    const float4 c0 = __ldg(a.camera_basis + 3 * view), c1 = __ldg(a.camera_basis + 3 * view + 1);
+    const float4 c2 = __ldg(a.camera_basis + 3 * view + 2);
+    PixelRay r;
+    r.world = view / a.cameras_per_world;
+    r.eye = mk3(c0.x, c0.y, c0.z);
+    const float3 right = mk3(c0.w, c1.x, c1.y), up = mk3(c1.z, c1.w, c2.x), fwd = mk3(c2.y, c2.z, c2.w);
+    r.d = a.sample > 0 ? picture_ray<true>(a, x, y, p, a.width, a.height, a.aspect, right, up, fwd, r.rng)
+                       : picture_ray<false>(a, x, y, p, a.width, a.height, a.aspect, right, up, fwd, r.rng);
+    return r;
+}
+
+// Light `lt` sampled from a hit, as trace does it: always two draws, then the way to the light and what arrives.
+struct LightSample {
+    float3 dir;
+    float distance, strength;
+};
+__device__ __forceinline__ LightSample sample_light(const DevLight &lt, float3 point, uint32_t &rng) {
+    const float z = 1.0f - 2.0f * rand_float(rng);
+    const float rad = sqrtf(fmaxf(0.0f, 1.0f - z * z));
+    const float phi = 6.28318530718f * rand_float(rng);
+    const float3 lp = lt.position + mk3(rad * cosf(phi), rad * sinf(phi), z) * lt.radius;
+    const float3 to_light = lp - point;
+    LightSample r;
+    r.distance = sqrtf(dot(to_light, to_light));
+    r.dir = to_light * recip(r.distance);
+    r.strength = lt.intensity * light_factor(lt, r.dir, r.distance);
+    return r;
+}
+
+// The picture hit of pixel p resolved to its surface.
+struct Surface {
+    float3 point, normal;
+    DevMaterial mat;
+};
+__device__ __forceinline__ Surface surface_of(const SceneParams &s, const PixelRay &r, int code, float4 h) {
+    Surface f;
+    int object;
+    f.point = r.eye + r.d * h.x;
+    resolve(s, r.world, f.point, r.d, code >= 0 ? code : -1, __float_as_int(h.w), h.y, h.z,
+        code <= CODE_SPHERE ? CODE_SPHERE - code : -1, code == CODE_FLOOR, f.normal, f.mat, object);
+    return f;
+}
+
+// The shadow rays of light a.light, one thread per pixel: bit a.light of visible set where the light reaches the hit as
+// far as spheres and the floor go, and the ray left for the shadow kernel where the light would add anything.
+__global__ void __launch_bounds__(256, 4) light_kernel(const __grid_constant__ SceneParams s, const RenderArgs a,
+    long long pixels) {
+    for (long long p = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; p < pixels;
+         p += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const int code = a.pic_code[p];
+        float reach = 0.0f;
+        unsigned visible = a.light == 0 ? 0u : a.visible[p];
+        if (code != CODE_NONE) {
+            PixelRay r = pixel_ray(a, p);
+            const float4 h = a.pic_hit[p];
+            const Surface f = surface_of(s, r, code, h);
+            for (int k = 0; k < 2 * a.light; ++k) rand_float(r.rng);
+            const DevLight &lt = s.lights[a.light];
+            const LightSample l = sample_light(lt, f.point, r.rng);
+            if (!(l.strength <= 0.0f)) {
+                const float3 so = offset_origin(f.point, f.normal, l.dir);
+                bool blocked = false;
+                for (int i = 0; i < s.sphere_count && !blocked; ++i) {
+                    float t;
+                    if (sphere_hit(s.spheres[i], so, l.dir, t) && t < l.distance) blocked = true;
+                }
+                if (!blocked) {
+                    float dd;
+                    blocked = floor_hit(s.floor, so, l.dir, l.distance, dd);
+                }
+                if (!blocked) {
+                    visible |= 1u << a.light;
+                    // Behind the surface the light adds only its highlight, which mostly rounds to nothing: adding
+                    // zeros changes nothing, so such a ray needs no answer.
+                    const float3 lit = lt.color * l.strength;
+                    bool adds = dot(l.dir, f.normal) > 0.0f;
+                    if (!adds) {
+                        const float3 spec = lit * powf(fmaxf(0.0f, dot(reflect(l.dir, f.normal), r.d)), f.mat.exponent);
+                        const float3 diff = lit * fmaxf(0.0f, dot(l.dir, f.normal));
+                        adds = !(spec.x == 0.0f && spec.y == 0.0f && spec.z == 0.0f && diff.x == 0.0f && diff.y == 0.0f &&
+                            diff.z == 0.0f);
+                    }
+                    if (adds) {
+                        reach = l.distance;
+                        int self = -1;
+                        if (code >= 0) {
+                            if (dot(l.dir, f.normal) < 0.0f) self = code * 4 + 2;
+                            else if (shadow_misses_own_mesh(s, r.world, code, __float_as_int(h.w), h.y, h.z, r.d, f.normal,
+                                         l.dir, f.point))
+                                self = code * 4 + 1;
+                        }
+                        a.shadow_self[p] = self;
+                        a.shadow_o[p] = make_float4(so.x, so.y, so.z, reach);
+                        a.shadow_d[p] = make_float4(l.dir.x, l.dir.y, l.dir.z, 0.0f);
+                    }
+                }
+            }
+        }
+        a.visible[p] = static_cast<uint8_t>(visible);
+        if (!(reach > 0.0f)) a.shadow_o[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+}
+
+// A finished sample of pixel p: added to the pixel's sum, which after the last sample becomes its average's bytes or, in
+// a single-view render, its radiance (render_pixel_rgb8, src/render_core.h:275-283).
+__device__ __forceinline__ void finish_sample(const SceneParams &s, const RenderArgs &a, long long p, float3 radiance,
+    uint32_t rng) {
+    float3 sum = mk3(0.0f, 0.0f, 0.0f);
+    if (a.sample > 0) {
+        const float4 before = a.sample_sum[p];
+        sum = mk3(before.x, before.y, before.z);
+    }
+    sum = sum + radiance;
+    if (a.sample + 1 < a.spp) {
+        a.sample_sum[p] = make_float4(sum.x, sum.y, sum.z, 0.0f);
+        a.rng_out[p] = rng;
+        return;
+    }
+    sum = sum * (1.0f / static_cast<float>(a.spp));
+    if (a.radiance) {
+        a.radiance[p] = make_float4(sum.x, sum.y, sum.z, 0.0f);
+    } else {
+        put_rgb(a.rgb, p, srgb_byte(s.srgb_table, sum.x) | (srgb_byte(s.srgb_table, sum.y) << 8) |
+            (srgb_byte(s.srgb_table, sum.z) << 16));
+    }
+}
+
+// Appends p to a list by the lanes that come here together: one atomic for all of them.
+__device__ __forceinline__ void append(int *list, int *count, int p) {
+    const unsigned here = __activemask();
+    const int lane = threadIdx.x & 31, leader = __ffs(here) - 1;
+    int at = 0;
+    if (lane == leader) at = atomicAdd(count, __popc(here));
+    list[__shfl_sync(here, at, leader) + __popc(here & ((1u << lane) - 1u))] = p;
+}
+
+// The sample's light at each hit, one thread per pixel (trace's first bounce). A path that goes on from a mirror is left in
+// the hand-over arrays (shadow_o: origin and throughput, shadow_d: direction, pic_hit: radiance so far) and its
+// pixel appended to the list (shadow_self).
+__global__ void __launch_bounds__(256, 4) finish_kernel(const __grid_constant__ SceneParams s, const RenderArgs a,
+    long long pixels) {
+    const float3 zero = mk3(0.0f, 0.0f, 0.0f);
+    for (long long p = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; p < pixels;
+         p += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const int code = a.pic_code[p];
+        PixelRay r = pixel_ray(a, p);
+        float3 radiance = zero;
+        if (code == CODE_NONE) {
+            const float t = saturate(dot(r.d, s.env_up) * 0.5f + 0.5f);
+            const float3 sky = (s.env_color_down + (s.env_color_up - s.env_color_down) * t) * s.env_intensity;
+            radiance = radiance + sky * 1.0f;
+        } else {
+            const Surface f = surface_of(s, r, code, a.pic_hit[p]);
+            const unsigned visible = s.light_count > 0 ? a.visible[p] : 0u;
+            float3 diffuse = zero, specular = zero;
+            for (int i = 0; i < s.light_count; ++i) {
+                const DevLight &lt = s.lights[i];
+                const LightSample l = sample_light(lt, f.point, r.rng);
+                if (!(visible >> i & 1u)) continue;
+                const float3 lit = lt.color * l.strength;
+                diffuse = diffuse + lit * fmaxf(0.0f, dot(l.dir, f.normal));
+                specular = specular + lit * powf(fmaxf(0.0f, dot(reflect(l.dir, f.normal), r.d)), f.mat.exponent);
+            }
+            const float3 direct = f.mat.diffuse_color * (diffuse * f.mat.kd) + specular * f.mat.ks;
+            radiance = radiance + (direct + f.mat.diffuse_color * (s.ambient * f.mat.kd)) * 1.0f;
+            const float throughput = 1.0f * f.mat.kr;
+            if (!(throughput < 1e-3f)) {
+                const float3 dir = reflect(r.d, f.normal), origin = offset_origin(f.point, f.normal, dir);
+                a.shadow_o[p] = make_float4(origin.x, origin.y, origin.z, throughput);
+                a.shadow_d[p] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(r.rng));
+                a.pic_hit[p] = make_float4(radiance.x, radiance.y, radiance.z, 0.0f);
+                append(a.shadow_self, a.bounces, static_cast<int>(p));
+                continue;
+            }
+        }
+        finish_sample(s, a, p, radiance, r.rng);
+    }
+}
+
+// The paths that go on from a mirror at the first hit, a thread each from the list, bounce after bounce to their end (trace
+// from depth 1 on): the closest hit, then light by light the shadow ray, each lane walking for itself (lane_walk).
+// What bounds this is the longest path's chain of walks (about 30 us a walk when a warp has a core to itself), not
+// their number, so the bounces stay in one launch and few paths are spread over all resident warps, a part of each
+// one's lanes. On 75,000 paths of two lights: 0.23 ms; a launch per bounce 0.45 (each waits for its own longest
+// path), a launch per bounce as packets 1.0 (rays off curved mirrors visit the union of a warp's nodes).
+template <int THREADS, int MIN_BLOCKS>
+__global__ void __launch_bounds__(THREADS, MIN_BLOCKS) bounce_kernel(const __grid_constant__ SceneParams s, const RenderArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int max_steps = s.blas_node_count + 2;
+    const int n = *a.bounces, per_view = a.width * a.rows;
+    const float3 zero = mk3(0.0f, 0.0f, 0.0f);
+    const int warps = gridDim.x * (THREADS / 32);
+    int width = 4;
+    while (width < 32 && width * warps < n) width *= 2;
+    if (lane >= width) return;
+    for (int at = (blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5)) * width + lane; at < n; at += warps * width) {
+        const int p = a.shadow_self[at];
+        const float4 o4 = a.shadow_o[p], d4 = a.shadow_d[p], r4 = a.pic_hit[p];
+        float3 o = xyz(o4), d = xyz(d4), radiance = xyz(r4);
+        float throughput = o4.w;
+        const int world = p / per_view / a.cameras_per_world;
+        uint32_t rng = __float_as_uint(d4.w);
+        for (int depth = 1;; ++depth) {
+            int best_sphere = -1, hit_inst = -1, hit_tri = -1;
+            bool hit_floor = false;
+            float tmax = 0.0f, hu = 0.0f, hv = 0.0f;
+            if (depth <= 4) {
+                tmax = spheres_and_floor(s, o, d, best_sphere, hit_floor);
+                lane_walk<false>(s, world, o, d, tmax, hit_inst, hit_tri, hu, hv, -1, max_steps, a.error_flag);
+            }
+            if (hit_inst < 0 && best_sphere < 0 && !hit_floor) {
+                const float t = saturate(dot(d, s.env_up) * 0.5f + 0.5f);
+                const float3 sky = (s.env_color_down + (s.env_color_up - s.env_color_down) * t) * s.env_intensity;
+                radiance = radiance + sky * throughput;
+                break;
+            }
+            const float3 point = o + d * tmax;
+            float3 normal, diffuse = zero, specular = zero;
+            DevMaterial mat;
+            int object;
+            resolve(s, world, point, d, hit_inst, hit_tri, hu, hv, best_sphere, hit_floor, normal, mat, object);
+            for (int i = 0; i < s.light_count; ++i) {
+                const DevLight &lt = s.lights[i];
+                const LightSample l = sample_light(lt, point, rng);
+                if (l.strength <= 0.0f) continue;
+                const float3 so = offset_origin(point, normal, l.dir);
+                bool blocked = false;
+                for (int k = 0; k < s.sphere_count && !blocked; ++k) {
+                    float t;
+                    if (sphere_hit(s.spheres[k], so, l.dir, t) && t < l.distance) blocked = true;
+                }
+                float dd;
+                if (blocked || floor_hit(s.floor, so, l.dir, l.distance, dd)) continue;
+                const int skip = hit_inst >= 0 && !(dot(l.dir, normal) < 0.0f) &&
+                        shadow_misses_own_mesh(s, world, hit_inst, hit_tri, hu, hv, d, normal, l.dir, point)
+                    ? hit_inst : -1;
+                float t = l.distance, u, v;
+                int by = -1, by_tri;
+                lane_walk<true>(s, world, so, l.dir, t, by, by_tri, u, v, skip, max_steps, a.error_flag);
+                if (by >= 0) continue;
+                const float3 lit = lt.color * l.strength;
+                diffuse = diffuse + lit * fmaxf(0.0f, dot(l.dir, normal));
+                specular = specular + lit * powf(fmaxf(0.0f, dot(reflect(l.dir, normal), d)), mat.exponent);
+            }
+            const float3 direct = mat.diffuse_color * (diffuse * mat.kd) + specular * mat.ks;
+            radiance = radiance + (direct + mat.diffuse_color * (s.ambient * mat.kd)) * throughput;
+            throughput *= mat.kr;
+            if (throughput < 1e-3f) break;
+            d = reflect(d, normal);
+            o = offset_origin(point, normal, d);
+        }
+        finish_sample(s, a, p, radiance, rng);
+    }
+}
+
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     // Every SM full of resident warps, and no more warps than there are fetches of tiles.
     long long blocks = static_cast<long long>(sms) * per_sm;
     const long long needed = (tiles + fetch * (threads / 32) - 1) / (fetch * (threads / 32));
     if (blocks > needed) blocks = needed;
-    e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
-    kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(s, a, counter, tiles, tiles_x, tiles_per_view, fetch);
+    kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(s, a, reinterpret_cast<int *>(counter), tiles, tiles_x,
+        tiles_per_view, fetch);
     return cudaGetLastError();
 }
 
 template <int THREADS, int MIN_BLOCKS, int CAP>
-cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, int *counter, const PersistentTuning &t,
-    cudaStream_t stream, cudaEvent_t after_camera, cudaEvent_t after_shade) {
+cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, unsigned long long *counters,
+    const PersistentTuning &t, cudaStream_t stream, cudaEvent_t after_camera, cudaEvent_t after_shade) {
     const int fetch = t.tile_fetch;
     const int tiles_x = (a.width + TILE_W - 1) / TILE_W, tiles_y = (a.rows + TILE_H - 1) / TILE_H;
     const int tiles_per_view = tiles_x * tiles_y;
@@ -1101,7 +1475,9 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, int *count
         mark(after_shade);
         return e;
     }
-    if (!a.basis_given) e = launch_prepare_cameras(a.cameras, a.views, a.camera_basis, stream);
+    // One fill zeroes every launch's queue counter.
+    e = cudaMemsetAsync(counters, 0, tile_counters(a, s.light_count) * sizeof(unsigned long long), stream);
+    if (e == cudaSuccess && !a.basis_given) e = launch_prepare_cameras(a.cameras, a.views, a.camera_basis, stream);
     if constexpr (CAP > 0) {
         if (e == cudaSuccess && a.views > 0) {
             view_order_kernel<CAP><<<static_cast<unsigned>(a.views), 128, 0, stream>>>(s, a);
@@ -1113,10 +1489,10 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, int *count
     if (e == cudaSuccess && paired) {
         const int ptx = (a.width + 3) / 4, pty = (a.rows + 3) / 4;
         const long long pair_tiles = a.view_info ? a.total_pair_tiles : static_cast<long long>(ptx) * pty * a.views;
-        e = launch_tiles(camera_tiles_kernel<THREADS, MIN_BLOCKS, CAP, true>, THREADS, s, a, counter, pair_tiles, ptx,
+        e = launch_tiles(camera_tiles_kernel<THREADS, MIN_BLOCKS, CAP, true>, THREADS, s, a, counters, pair_tiles, ptx,
             ptx * pty, fetch, stream);
     } else if (e == cudaSuccess) {
-        e = launch_tiles(camera_tiles_kernel<THREADS, MIN_BLOCKS, CAP, false>, THREADS, s, a, counter, tiles, tiles_x,
+        e = launch_tiles(camera_tiles_kernel<THREADS, MIN_BLOCKS, CAP, false>, THREADS, s, a, counters, tiles, tiles_x,
             tiles_per_view, fetch, stream);
     }
     mark(after_camera);
@@ -1131,20 +1507,61 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, int *count
     if (e != cudaSuccess) return e;
     long long blocks = (pixels + 255) / 256;
     if (blocks > 32LL * sms) blocks = 32LL * sms;
-    if (a.radiance) shade_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(s, a, pixels);
-    else shade_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(s, a, pixels);
+    auto shadows = [&](const RenderArgs &args, unsigned long long *counter) {
+        // Worlds too large for candidate lists: the shadow rays as warp packets over the world's tree (0.39 against
+        // 0.41 ms as persistent-kernel jobs with lane refill on the large world's 1280 x 720 frame).
+        auto run = [&](auto kernel) {
+            return launch_tiles(kernel, THREADS, s, args, counter, tiles, tiles_x, tiles_per_view, fetch, stream);
+        };
+        if constexpr (CAP == 0)
+            return args.visible ? run(shadow_packets_kernel<THREADS, MIN_BLOCKS, true>)
+                                : run(shadow_packets_kernel<THREADS, MIN_BLOCKS, false>);
+        else
+            return args.visible ? run(shadow_tiles_kernel<THREADS, MIN_BLOCKS, CAP, true>)
+                                : run(shadow_tiles_kernel<THREADS, MIN_BLOCKS, CAP, false>);
+    };
+    if (!one_pass(a, s.light_count)) {
+        RenderArgs b = a;
+        unsigned long long *counter = counters;
+        for (b.sample = 0; b.sample < a.spp && e == cudaSuccess; ++b.sample) {
+            if (b.sample > 0) {
+                b.rng_in = a.rng_out;
+                b.depth = b.normal = nullptr;
+                b.object_id = b.hit_instance = nullptr;
+                e = launch_tiles(camera_tiles_kernel<THREADS, MIN_BLOCKS, CAP, false, true>, THREADS, s, b, counter, tiles, tiles_x,
+                    tiles_per_view, fetch, stream);
+            }
+            ++counter;
+            for (b.light = 0; b.light < s.light_count && e == cudaSuccess; ++b.light) {
+                light_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(s, b, pixels);
+                e = cudaGetLastError();
+                if (e == cudaSuccess) e = shadows(b, counter);
+                ++counter;
+            }
+            if (e != cudaSuccess) return e;
+            b.light = 0;
+            b.bounces = reinterpret_cast<int *>(counter);
+            finish_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(s, b, pixels);
+            if (a.reflective) {
+                constexpr int THREADS_B = 128, PER_SM = 4;
+                long long groups = (pixels + THREADS_B / 32 - 1) / (THREADS_B / 32);
+                if (groups > static_cast<long long>(PER_SM) * sms) groups = static_cast<long long>(PER_SM) * sms;
+                bounce_kernel<THREADS_B, PER_SM><<<static_cast<unsigned>(groups), THREADS_B, 0, stream>>>(s, b);
+            }
+            ++counter;
+            e = cudaGetLastError();
+        }
+        mark(after_shade);
+        return e;
+    }
+    blocks = (pixels + 127) / 128;
+    if (blocks > 64LL * sms) blocks = 64LL * sms;
+    if (a.radiance) shade_kernel<true><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(s, a, pixels);
+    else shade_kernel<false><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(s, a, pixels);
     e = cudaGetLastError();
     mark(after_shade);
     if (e != cudaSuccess || s.light_count != 1) return e;
-    // Worlds too large for candidate lists: the shadow rays as warp packets over the world's tree (0.39 against
-    // 0.41 ms as persistent-kernel jobs with lane refill on the large world's 1280 x 720 frame).
-    if constexpr (CAP == 0) {
-        return launch_tiles(shadow_packets_kernel<THREADS, MIN_BLOCKS>, THREADS, s, a, counter, tiles, tiles_x,
-            tiles_per_view, fetch, stream);
-    } else {
-        return launch_tiles(shadow_tiles_kernel<THREADS, MIN_BLOCKS, CAP>, THREADS, s, a, counter, tiles, tiles_x,
-            tiles_per_view, fetch, stream);
-    }
+    return shadows(a, counters + 1);
 }
 
 }  // namespace
@@ -1170,7 +1587,7 @@ cudaError_t launch_rays_packets(const SceneParams &s, const RayArgs &r, int *cou
     return cudaGetLastError();
 }
 
-cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, int *counter, const PersistentTuning &t,
+cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, unsigned long long *counter, const PersistentTuning &t,
     cudaStream_t stream, cudaEvent_t after_camera, cudaEvent_t after_shade) {
     // (threads per CTA, register budget) -> the instantiation with that budget, and the candidate lists'
     // capacity: 32 for worlds of up to 32 instances, else TILE_MAX_INSTANCES; larger worlds walk their tree
