@@ -1146,7 +1146,14 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) ray_packets_kernel(const 
         float tmax = live ? spheres_and_floor(s, o, d, best_sphere, hit_floor) : 0.0f;
         int hit_inst = -1, hit_tri = -1;
         float hu = 0.0f, hv = 0.0f;
-        packet_walk<false>(s, sm, lane, world, live, o, d, tmax, hit_inst, hit_tri, hu, hv, -1, max_steps, r.error_flag);
+        // A packet pays while its rays look the same way: it visits the nodes that any of them enters. Rays spread over
+        // more than a half space around the middle one walk each for themselves (1024 worlds of 20 instances, 720
+        // rays in all directions: 0.245 against 0.35 ms as packets; a 720-beam scan 0.13 against 0.17 ms).
+        const float3 middle = mk3(__shfl_sync(FULL, d.x, 16), __shfl_sync(FULL, d.y, 16), __shfl_sync(FULL, d.z, 16));
+        if (__all_sync(FULL, !live || dot(d, middle) > 0.0f))
+            packet_walk<false>(s, sm, lane, world, live, o, d, tmax, hit_inst, hit_tri, hu, hv, -1, max_steps, r.error_flag);
+        else if (live)
+            lane_walk<false>(s, world, o, d, tmax, hit_inst, hit_tri, hu, hv, -1, max_steps, r.error_flag);
         if (!valid) continue;
         const bool found = live && (hit_inst >= 0 || best_sphere >= 0 || hit_floor) && tmax <= r.max_distance;
         float3 normal = mk3(0.0f, 0.0f, 0.0f);
@@ -1161,13 +1168,6 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) ray_packets_kernel(const 
     }
 }
 
-template <class Kernel>
-cudaError_t launch_tiles(Kernel kernel, int threads, const SceneParams &s, const RenderArgs &a,
-    unsigned long long *counter, long long tiles, int tiles_x, int tiles_per_view, int fetch, cudaStream_t stream) {
-    int device = 0, sms = 0, per_sm = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
 // ------------------------------------------------------------------------------------------------------
 // Sample passes: pictures of several samples per pixel, several lights, or mirrors, on the same tile kernels. Per sample:
 // the camera kernel (its picture rays only after the first sample), then for each light a light_kernel that leaves
@@ -1447,6 +1447,13 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) bounce_kernel(const __gri
     }
 }
 
+template <class Kernel>
+cudaError_t launch_tiles(Kernel kernel, int threads, const SceneParams &s, const RenderArgs &a,
+    unsigned long long *counter, long long tiles, int tiles_x, int tiles_per_view, int fetch, cudaStream_t stream) {
+    int device = 0, sms = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     // Every SM full of resident warps, and no more warps than there are fetches of tiles.
