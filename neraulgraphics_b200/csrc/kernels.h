@@ -35,6 +35,7 @@ struct BuildArgs {
     int *roots;                    // worlds
     int *parent;                   // 2n - 1; parent[0] stays -1
     int *arrivals;                 // n - 1 counters, zero between builds
+    int *built;                    // a counter, zero between builds: the per-world build's finished CTAs; or null
     int *error_flag;               // set nonzero if a climb runs longer than any valid tree allows
     float4 *tlas_pairs;            // (n - 1) x 4 child-pair records of the internal nodes, or null
     // Worlds of uneven sizes (the per-world build only; per_world is then the largest): world w's instances
@@ -63,6 +64,11 @@ struct LargeBuildScratch {
 };
 int large_sort_blocks(long long n);
 cudaError_t launch_build_large(const BuildArgs &a, const LargeBuildScratch &t, cudaStream_t stream);
+
+// Nanoseconds of the GPU's global timer, and the render that they belong to once they are whole.
+struct RenderTimes {
+    unsigned long long begin, shade, shadow, end, id;
+};
 
 // Rendering every view of a batch.
 struct RenderArgs {
@@ -120,6 +126,11 @@ struct RenderArgs {
     uint8_t *visible;              // per pixel: bit i set while light i is not found blocked
     int light;                     // the light whose shadow rays this pass traces
     int *bounces;                  // how many pixels' paths go on from a mirror
+    // The render's GPU times, taken by its kernels (null: not timed): when it, its shading and its shadow rays began and
+    // when its last kernel's last warp ended.
+    RenderTimes *times;
+    unsigned long long *ended;     // zeroed: the warps of the last kernel that have ended
+    unsigned long long time_id;    // what the last warp leaves in times->id
 };
 
 // The running average of a single-view renderer's pictures (render_pixel, src/render_core.h:288-301): per pixel
@@ -172,11 +183,11 @@ cudaError_t launch_rays_packets(const SceneParams &s, const RayArgs &r, int *cou
 constexpr int TILE_MAX_INSTANCES = 256;  // the largest world rendered from candidate lists
 inline bool one_pass(const RenderArgs &a, int lights) { return a.spp == 1 && lights <= 1 && !a.reflective; }
 inline size_t tile_counters(const RenderArgs &a, int lights) {
-    return !a.rgb ? 1 : one_pass(a, lights) ? 2 : static_cast<size_t>(a.spp) * (2 + lights);
+    // One more counts the ended warps of the last kernel of a render that is timed by its kernels.
+    return 1 + (!a.rgb ? 1 : one_pass(a, lights) ? 2 : static_cast<size_t>(a.spp) * (2 + lights));
 }
-// after_camera / after_shade (may be null) are recorded on the stream after the camera and shade kernels.
 cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, unsigned long long *counters, const PersistentTuning &t,
-    cudaStream_t stream, cudaEvent_t after_camera, cudaEvent_t after_shade);
+    cudaStream_t stream);
 
 // The adjoint of the depth and normal images (see adjoint.cu). Every pointer is device memory; grad_normal
 // may be null; the gradients are added to grad_matrices and grad_cameras.

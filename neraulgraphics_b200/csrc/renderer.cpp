@@ -221,7 +221,11 @@ struct Renderer {
     bool cuda_touched = false;  // set before the first CUDA call of the constructor
     cudaStream_t own_stream = nullptr, stream = nullptr;
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr, ev_done = nullptr;
-    cudaEvent_t ev_stage[2] = {nullptr, nullptr};  // between the tile render's camera, shade and shadow kernels
+    // The tile render's times, taken by its own kernels (an event between two kernels costs a small render 2.5 us), and
+    // their copy for the host. times_id: the render whose times are asked for, 0 when the events have them.
+    DevBuf<RenderTimes> times;
+    RenderTimes *host_times = nullptr;  // pinned
+    unsigned long long times_id = 0, times_count = 0;
     int stages = 0;                                // kernels timed apart in the last render: 1 or 3
     float stage_ms[3] = {0.0f, 0.0f, 0.0f};
     bool synchronous = true;
@@ -254,6 +258,7 @@ struct Renderer {
     }
     bool use_large_build() const { return build_mode == 2 || (build_mode == 0 && per_world > MAX_PER_WORLD); }
     void wait(cudaEvent_t ev, double seconds);
+    void wait_times();
     void set_instance_transforms(const float *m, int memory);
     void bind_bodies(int bpw, const int32_t *boi, const float *lp, const float *sc);
     void set_body_poses(const float *poses, int memory);
@@ -350,8 +355,10 @@ void Renderer::init(const ngb_scene &s, const UnevenLayout *layout) {
     stream = own_stream;
     CK(cudaEventCreate(&ev_start));
     CK(cudaEventCreate(&ev_stop));
-    CK(cudaEventCreate(&ev_stage[0]));
-    CK(cudaEventCreate(&ev_stage[1]));
+    CK(cudaHostAlloc(&host_times, sizeof(RenderTimes), cudaHostAllocDefault));
+    *host_times = RenderTimes{};
+    times.ensure(1);
+    CK(cudaMemsetAsync(times.p, 0, sizeof(RenderTimes), stream));
     CK(cudaEventCreateWithFlags(&ev_done, cudaEventDisableTiming));
     CK(cudaHostAlloc(&host_error, sizeof(int), cudaHostAllocDefault));
     CK(cudaHostAlloc(&host_count, sizeof(int), cudaHostAllocDefault));
@@ -507,7 +514,7 @@ void Renderer::init(const ngb_scene &s, const UnevenLayout *layout) {
     roots.ensure(worlds);
     parent.ensure(2 * n - 1);
     leaf_of.ensure(n);
-    arrivals.ensure(std::max<long long>(n - 1, 1));
+    arrivals.ensure(std::max<long long>(n - 1, 1) + 1);  // and the build's count of finished CTAs
     CK(cudaMemset(parent.p, 0xFF, (2 * n - 1) * sizeof(int)));
     CK(cudaMemset(arrivals.p, 0, arrivals.n * sizeof(int)));
     params.tlas = tlas.p;
@@ -553,16 +560,15 @@ void Renderer::teardown() {
     if (own_stream) cudaStreamSynchronize(own_stream);
     if (ev_start) cudaEventDestroy(ev_start);
     if (ev_stop) cudaEventDestroy(ev_stop);
-    for (cudaEvent_t &e : ev_stage) {
-        if (e) cudaEventDestroy(e);
-        e = nullptr;
-    }
     if (ev_done) cudaEventDestroy(ev_done);
     if (host_error) cudaFreeHost(host_error);
     if (host_count) cudaFreeHost(host_count);
+    if (host_times) cudaFreeHost(host_times);
+    times.release();
     if (own_stream) cudaStreamDestroy(own_stream);
     ev_start = ev_stop = ev_done = nullptr;
     host_error = host_count = nullptr;
+    host_times = nullptr;
     own_stream = nullptr;
     // The DevBufs free themselves; the device must be current while they do, so release them here.
     blas.release(), tris.release(), attrs.release(), tri_index.release(), slot_blas_root.release();
@@ -606,20 +612,43 @@ void Renderer::wait(cudaEvent_t ev, double seconds) {
     }
 }
 
+// Waits, with the limit, until the last timed call's times are there.
+void Renderer::wait_times() {
+    if (!timing_pending) return;
+    if (times_id == 0) return wait(ev_stop, timeout);
+    const auto start = std::chrono::steady_clock::now();
+    for (;;) {
+        // Read aside of the stream the render was queued on, until its last warp has left its number.
+        CK(cudaMemcpyAsync(host_times, times.p, sizeof(RenderTimes), cudaMemcpyDeviceToHost, own_stream));
+        CK(cudaEventRecord(ev_done, own_stream));
+        wait(ev_done, timeout);
+        if (host_times->id == times_id) return;
+        if (std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count() > timeout)
+            throw Timeout("the GPU work did not finish within " + std::to_string(timeout) + " seconds");
+        std::this_thread::sleep_for(std::chrono::microseconds(20));
+    }
+}
+
 // Called after every launch: brings the device's error flag back with the work and, when synchronous,
 // waits for both.
 // The last launch's GPU times, once its events have completed.
 void Renderer::read_timing() {
-    if (!timing_pending) return;
-    CK(cudaEventElapsedTime(&kernel_ms, ev_start, ev_stop));
-    if (stages == 3) {
-        CK(cudaEventElapsedTime(&stage_ms[0], ev_start, ev_stage[0]));
-        CK(cudaEventElapsedTime(&stage_ms[1], ev_stage[0], ev_stage[1]));
-        CK(cudaEventElapsedTime(&stage_ms[2], ev_stage[1], ev_stop));
-    } else {
-        stage_ms[0] = kernel_ms;
-    }
+    if (!timing_pending || (times_id != 0 && host_times->id != times_id)) return;
     timing_pending = false;
+    if (times_id == 0) {
+        CK(cudaEventElapsedTime(&kernel_ms, ev_start, ev_stop));
+        stage_ms[0] = kernel_ms;
+        return;
+    }
+    auto ms = [](unsigned long long from, unsigned long long to) {
+        return to > from ? static_cast<float>(to - from) * 1e-6f : 0.0f;
+    };
+    const RenderTimes t = *host_times;
+    const unsigned long long shade = t.shade ? t.shade : t.end, shadow = t.shadow ? t.shadow : t.end;
+    kernel_ms = ms(t.begin, t.end);
+    stage_ms[0] = ms(t.begin, shade);
+    stage_ms[1] = ms(shade, shadow);
+    stage_ms[2] = ms(shadow, t.end);
 }
 
 // Queues the copy of the device error flag to host_error, for a wait that follows.
@@ -669,6 +698,7 @@ void Renderer::build(const float *matrices_in, int compose, const float *poses, 
     a.roots = roots.p;
     a.parent = parent.p;
     a.arrivals = arrivals.p;
+    a.built = arrivals.p + arrivals.n - 1;
     a.error_flag = error_flag.p;
     a.tlas_pairs = tlas_pairs.p;
     a.world_first = uneven ? world_first.p : nullptr;
@@ -1055,8 +1085,9 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         "reflective material");
     // Inside a CUDA graph capture the timing events would be graph nodes whose times cannot be read: the
     // render is then not timed (last_kernel_ms keeps the previous figure).
-    const bool timed = !capturing();
-    if (timed) CK(cudaEventRecord(ev_start, stream));
+    const bool timed = !capturing(), by_kernels = timed && tiles && single && !a.radiance && pixels() > 0 &&
+        (!a.rgb || params.light_count == 1);
+    if (timed && !by_kernels) CK(cudaEventRecord(ev_start, stream));
     if (tiles) {
         a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
         if (per_world > 0 && per_world <= TILE_MAX_INSTANCES) {
@@ -1083,9 +1114,16 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
             a.sample_sum = sample_sum.ensure(pixels());
             a.visible = sample_visible.ensure(pixels());
         }
-        CK(launch_render_tiles(params, a, work_counter.ensure(tile_counters(a, params.light_count)), tile_tuning, stream,
-            timed ? ev_stage[0] : nullptr, timed ? ev_stage[1] : nullptr));
-        stages = single ? 3 : 1;
+        const size_t counters = tile_counters(a, params.light_count);
+        work_counter.ensure(counters);
+        if (by_kernels) {
+            // The times of a render before this one that nobody read are given up: it writes the same place.
+            a.times = times.p;
+            a.ended = work_counter.p + counters - 1;
+            a.time_id = ++times_count;
+        }
+        CK(launch_render_tiles(params, a, work_counter.p, tile_tuning, stream));
+        stages = by_kernels ? 3 : 1;
     } else if (persistent) {
         a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
         CK(launch_render_persistent(params, a, reinterpret_cast<int *>(work_counter.p), tuning, stream));
@@ -1098,7 +1136,8 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         CK(launch_accumulate(a.radiance, view_accum.p, frame, static_cast<long long>(pixels()), srgb_table.p,
             view_argb.p, a.rgb, stream));
     if (timed) {
-        CK(cudaEventRecord(ev_stop, stream));
+        times_id = by_kernels ? a.time_id : 0;
+        if (!by_kernels) CK(cudaEventRecord(ev_stop, stream));
         timing_pending = true;
     }
     finish();
@@ -1149,6 +1188,7 @@ void Renderer::cast_rays(const float *o, const float *d, int rays_per_world, flo
         kernel_choice == 2 ? tuning : ray_tuning, stream));
     if (timed) {
         stages = 1;
+        times_id = 0;
         CK(cudaEventRecord(ev_stop, stream));
         timing_pending = true;
     }
@@ -1527,7 +1567,7 @@ float ngb_last_kernel_ms(const ngb_renderer *ch) {
     if (!h) return 0.0f;
     float ms = 0.0f;
     guarded(h, [&](ngb::Renderer &r) {
-        if (r.timing_pending) r.wait(r.ev_stop, r.timeout);
+        r.wait_times();
         r.read_timing();
         ms = r.kernel_ms;
     });
@@ -1537,7 +1577,7 @@ float ngb_last_kernel_ms(const ngb_renderer *ch) {
 int ngb_last_stage_ms(ngb_renderer *h, float *ms, int32_t capacity, int32_t *count) {
     return guarded(h, [&](ngb::Renderer &r) {
         ngb::require(ms != nullptr && count != nullptr && capacity >= 0, "ms and count must not be null");
-        if (r.timing_pending) r.wait(r.ev_stop, r.timeout);
+        r.wait_times();
         r.read_timing();
         *count = r.stages;
         for (int i = 0; i < r.stages && i < capacity; ++i) ms[i] = r.stage_ms[i];
@@ -1735,6 +1775,7 @@ int ngb_depth_normal_adjoint(ngb_renderer *h, const float *matrices, const float
         CK(cudaEventRecord(r.ev_start, r.stream));
         CK(ngb::launch_depth_normal_adjoint(r.params, a, r.stream));
         CK(cudaEventRecord(r.ev_stop, r.stream));
+        r.times_id = 0;
         r.stages = 1;
         r.timing_pending = true;
         r.finish();

@@ -547,38 +547,86 @@ __device__ __forceinline__ TileAt pair_tile_at(const RenderArgs &a, long long ti
     return t;
 }
 
-// One CTA per view: its world's instances in the order the view's tiles walk their candidates, nearest bound first
-// (the eye's distance to the instance's leaf box, 1e-5 under it: no camera ray of the view can enter the box
-// closer), ties by leaf order. The bound depends on the eye alone, so every tile of the view takes this order and
-// keeps only its own candidates.
-template <int CAP>
-__global__ void __launch_bounds__(128) view_order_kernel(const __grid_constant__ SceneParams s, const RenderArgs a) {
-    __shared__ float bound[CAP];
-    const int view = blockIdx.x;
-    const int world = view / a.cameras_per_world;
-    const int P = s.instance_count > 0 ? world_count_of(s, world) : 0;
-    const float4 c0 = __ldg(a.camera_basis + 3 * view);
-    const float3 eye = mk3(c0.x, c0.y, c0.z);
-    const float4 *leaves = world_leaves(s, world);
-    for (int j = threadIdx.x; j < P; j += blockDim.x) {
-        const float4 lo = __ldg(leaves + 2 * j), hi = __ldg(leaves + 2 * j + 1);
-        const float dx = fmaxf(fmaxf(lo.x - eye.x, eye.x - hi.x), 0.0f);
-        const float dy = fmaxf(fmaxf(lo.y - eye.y, eye.y - hi.y), 0.0f);
-        const float dz = fmaxf(fmaxf(lo.z - eye.z, eye.z - hi.z), 0.0f);
-        bound[j] = sqrtf(dx * dx + dy * dy + dz * dz) * 0.99999f;
+__device__ __forceinline__ unsigned long long now() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// A stage's beginning, by one thread of its launch.
+__device__ __forceinline__ void mark_begin(unsigned long long *at) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<volatile unsigned long long *>(at) = now();
+}
+// The end of a warp of the render's last kernel; the last of them leaves the time and the render's number.
+__device__ __forceinline__ void mark_end(const RenderArgs &a) {
+    if ((threadIdx.x & 31) != 0) return;
+    const unsigned long long warps = static_cast<unsigned long long>(gridDim.x) * (blockDim.x >> 5);
+    if (atomicAdd(a.ended, 1ull) + 1 == warps) {
+        *reinterpret_cast<volatile unsigned long long *>(&a.times->end) = now();
+        __threadfence();
+        *reinterpret_cast<volatile unsigned long long *>(&a.times->id) = a.time_id;
     }
-    __syncthreads();
-    int *order = a.view_order + static_cast<long long>(view) * a.order_stride;
-    float *order_bound = a.view_bound + static_cast<long long>(view) * a.order_stride;
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        const float bi = bound[i];
-        int rank = 0;
-        for (int k = 0; k < P; ++k) {
-            const float bk = bound[k];
-            rank += (bk < bi) || (bk == bi && k < i);
+}
+
+// The start of a render, one CTA per view: the launches' queue counters zeroed, the view's camera basis
+// (camera_from_matrix, src/render_core.h:264-273, renormalised) unless it is given, and its world's instances in the order
+// the view's tiles walk their candidates, nearest bound first (the eye's distance to the instance's leaf box, 1e-5
+// under it: no camera ray of the view can enter the box closer), ties by leaf order. The bound depends on the eye
+// alone, so every tile of the view takes this order and keeps only its own candidates. CAP 0: no order (worlds walked
+// as packets). One launch for what were a fill and two kernels: a small render's time is its launches' (2.5 us each).
+template <int CAP>
+__global__ void __launch_bounds__(128) setup_kernel(const __grid_constant__ SceneParams s, const RenderArgs a,
+    unsigned long long *counters, int counter_count) {
+    __shared__ float bound[CAP > 0 ? CAP : 1];
+    __shared__ float3 eye_shared;
+    const int view = blockIdx.x;
+    if (a.times && view == 0 && threadIdx.x == 0) {
+        volatile RenderTimes *t = a.times;
+        t->shade = t->shadow = 0;
+        t->begin = now();
+    }
+    if (view == 0)
+        for (int k = threadIdx.x; k < counter_count; k += blockDim.x) counters[k] = 0;
+    if (threadIdx.x == 0) {
+        if (a.basis_given) {
+            eye_shared = xyz(a.camera_basis[3 * view]);
+        } else {
+            float m[12];
+            for (int k = 0; k < 12; ++k) m[k] = a.cameras[12 * static_cast<size_t>(view) + k];
+            const float3 right = normalize(mk3(m[0], m[4], m[8]));
+            const float3 up = normalize(mk3(m[1], m[5], m[9]));
+            const float3 fwd = normalize(mk3(-m[2], -m[6], -m[10]));
+            a.camera_basis[3 * view] = make_float4(m[3], m[7], m[11], right.x);
+            a.camera_basis[3 * view + 1] = make_float4(right.y, right.z, up.x, up.y);
+            a.camera_basis[3 * view + 2] = make_float4(up.z, fwd.x, fwd.y, fwd.z);
+            eye_shared = mk3(m[3], m[7], m[11]);
         }
-        order[rank] = i;
-        order_bound[rank] = bi;
+    }
+    if constexpr (CAP > 0) {
+        __syncthreads();
+        const int world = view / a.cameras_per_world;
+        const int P = s.instance_count > 0 ? world_count_of(s, world) : 0;
+        const float3 eye = eye_shared;
+        const float4 *leaves = world_leaves(s, world);
+        for (int j = threadIdx.x; j < P; j += blockDim.x) {
+            const float4 lo = leaves[2 * j], hi = leaves[2 * j + 1];
+            const float dx = fmaxf(fmaxf(lo.x - eye.x, eye.x - hi.x), 0.0f);
+            const float dy = fmaxf(fmaxf(lo.y - eye.y, eye.y - hi.y), 0.0f);
+            const float dz = fmaxf(fmaxf(lo.z - eye.z, eye.z - hi.z), 0.0f);
+            bound[j] = sqrtf(dx * dx + dy * dy + dz * dz) * 0.99999f;
+        }
+        __syncthreads();
+        int *order = a.view_order + static_cast<long long>(view) * a.order_stride;
+        float *order_bound = a.view_bound + static_cast<long long>(view) * a.order_stride;
+        for (int i = threadIdx.x; i < P; i += blockDim.x) {
+            const float bi = bound[i];
+            int rank = 0;
+            for (int k = 0; k < P; ++k) {
+                const float bk = bound[k];
+                rank += (bk < bi) || (bk == bi && k < i);
+            }
+            order[rank] = i;
+            order_bound[rank] = bi;
+        }
     }
 }
 
@@ -625,7 +673,10 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) camera_tiles_kernel(const
     const float fs = a.fov_scale;
     for (;;) {
         const long long first = fetch_tiles(counter, lane, fetch);
-        if (first >= tiles) break;
+        if (first >= tiles) {
+            if (!LATER && a.times && !a.rgb) mark_end(a);
+            break;
+        }
         const long long last = first + fetch < tiles ? first + fetch : tiles;
         for (long long tile = first; tile < last; ++tile) {
             const TileAt T = PAIRED ? pair_tile_at(a, tile, tiles_x, tiles_per_view, lane)
@@ -814,6 +865,7 @@ __global__ void __launch_bounds__(128, 8) shade_kernel(const __grid_constant__ S
     long long pixels) {
     const long long per_view = static_cast<long long>(a.width) * a.rows;
     const float3 zero = mk3(0.0f, 0.0f, 0.0f);
+    if (a.times) mark_begin(&a.times->shade);
     for (long long p = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; p < pixels;
          p += static_cast<long long>(gridDim.x) * blockDim.x) {
         int view, rem, row0 = 0, width = a.width, height = a.height;
@@ -957,9 +1009,13 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_tiles_kernel(const
     const int max_steps = s.blas_node_count + 2;
     const DevLight &lt = s.lights[BITS ? a.light : 0];
     const float INF = __int_as_float(0x7f800000);
+    if (!BITS && a.times) mark_begin(&a.times->shadow);
     for (;;) {
         const long long first = fetch_tiles(counter, lane, fetch);
-        if (first >= tiles) break;
+        if (first >= tiles) {
+            if (!BITS && a.times) mark_end(a);
+            break;
+        }
         const long long last = first + fetch < tiles ? first + fetch : tiles;
         for (long long tile = first; tile < last; ++tile) {
             const TileAt T = tile_at(a, tile, tiles_x, tiles_per_view, lane);
@@ -1078,9 +1134,13 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_packets_kernel(con
     WarpSmem<0> &sm = warp_smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int max_steps = s.blas_node_count + 2;
+    if (!BITS && a.times) mark_begin(&a.times->shadow);
     for (;;) {
         const long long first = fetch_tiles(counter, lane, fetch);
-        if (first >= tiles) break;
+        if (first >= tiles) {
+            if (!BITS && a.times) mark_end(a);
+            break;
+        }
         const long long last = first + fetch < tiles ? first + fetch : tiles;
         for (long long tile = first; tile < last; ++tile) {
             const TileAt T = tile_at(a, tile, tiles_x, tiles_per_view, lane);
@@ -1467,30 +1527,17 @@ cudaError_t launch_tiles(Kernel kernel, int threads, const SceneParams &s, const
 
 template <int THREADS, int MIN_BLOCKS, int CAP>
 cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, unsigned long long *counters,
-    const PersistentTuning &t, cudaStream_t stream, cudaEvent_t after_camera, cudaEvent_t after_shade) {
+    const PersistentTuning &t, cudaStream_t stream) {
     const int fetch = t.tile_fetch;
     const int tiles_x = (a.width + TILE_W - 1) / TILE_W, tiles_y = (a.rows + TILE_H - 1) / TILE_H;
     const int tiles_per_view = tiles_x * tiles_y;
     const long long tiles = a.view_info ? a.total_tiles : static_cast<long long>(tiles_per_view) * a.views;
     const bool aov = a.depth || a.normal || a.object_id || a.hit_instance;
     cudaError_t e = cudaSuccess;
-    auto mark = [&](cudaEvent_t ev) {
-        if (e == cudaSuccess && ev) e = cudaEventRecord(ev, stream);
-    };
-    if (tiles == 0 || (!a.rgb && !aov)) {
-        mark(after_camera);
-        mark(after_shade);
-        return e;
-    }
-    // One fill zeroes every launch's queue counter.
-    e = cudaMemsetAsync(counters, 0, tile_counters(a, s.light_count) * sizeof(unsigned long long), stream);
-    if (e == cudaSuccess && !a.basis_given) e = launch_prepare_cameras(a.cameras, a.views, a.camera_basis, stream);
-    if constexpr (CAP > 0) {
-        if (e == cudaSuccess && a.views > 0) {
-            view_order_kernel<CAP><<<static_cast<unsigned>(a.views), 128, 0, stream>>>(s, a);
-            e = cudaGetLastError();
-        }
-    }
+    if (tiles == 0 || (!a.rgb && !aov)) return e;
+    setup_kernel<CAP><<<static_cast<unsigned>(a.views), 128, 0, stream>>>(s, a, counters,
+        static_cast<int>(tile_counters(a, s.light_count)));
+    e = cudaGetLastError();
     // Both kinds of camera ray: paired 4 x 4 tiles (pair_tile_at).
     const bool paired = t.tile_pairs && a.rgb && aov && (!a.view_info || a.view_pair_tile);
     if (e == cudaSuccess && paired) {
@@ -1502,11 +1549,7 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, unsigned l
         e = launch_tiles(camera_tiles_kernel<THREADS, MIN_BLOCKS, CAP, false>, THREADS, s, a, counters, tiles, tiles_x,
             tiles_per_view, fetch, stream);
     }
-    mark(after_camera);
-    if (e != cudaSuccess || !a.rgb) {
-        mark(after_shade);
-        return e;
-    }
+    if (e != cudaSuccess || !a.rgb) return e;
     const long long pixels = a.view_info ? a.total_pixels : static_cast<long long>(a.views) * a.width * a.rows;
     int device = 0, sms = 0;
     e = cudaGetDevice(&device);
@@ -1558,7 +1601,6 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, unsigned l
             ++counter;
             e = cudaGetLastError();
         }
-        mark(after_shade);
         return e;
     }
     blocks = (pixels + 127) / 128;
@@ -1566,7 +1608,6 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, unsigned l
     if (a.radiance) shade_kernel<true><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(s, a, pixels);
     else shade_kernel<false><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(s, a, pixels);
     e = cudaGetLastError();
-    mark(after_shade);
     if (e != cudaSuccess || s.light_count != 1) return e;
     return shadows(a, counters + 1);
 }
@@ -1595,34 +1636,34 @@ cudaError_t launch_rays_packets(const SceneParams &s, const RayArgs &r, int *cou
 }
 
 cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, unsigned long long *counter, const PersistentTuning &t,
-    cudaStream_t stream, cudaEvent_t after_camera, cudaEvent_t after_shade) {
+    cudaStream_t stream) {
     // (threads per CTA, register budget) -> the instantiation with that budget, and the candidate lists'
     // capacity: 32 for worlds of up to 32 instances, else TILE_MAX_INSTANCES; larger worlds walk their tree
     // as a packet (capacity 0).
     if (s.instance_count > 0 && s.per_world > TILE_MAX_INSTANCES) {
-        if (t.threads == 128 && t.registers == 64) return launch_variant<128, 8, 0>(s, a, counter, t, stream, after_camera, after_shade);
-        if (t.threads == 128 && t.registers == 56) return launch_variant<128, 9, 0>(s, a, counter, t, stream, after_camera, after_shade);
-        if (t.threads == 128 && t.registers == 48) return launch_variant<128, 10, 0>(s, a, counter, t, stream, after_camera, after_shade);
-        if (t.threads == 128 && t.registers == 80) return launch_variant<128, 6, 0>(s, a, counter, t, stream, after_camera, after_shade);
-        if (t.threads == 256 && t.registers == 64) return launch_variant<256, 4, 0>(s, a, counter, t, stream, after_camera, after_shade);
+        if (t.threads == 128 && t.registers == 64) return launch_variant<128, 8, 0>(s, a, counter, t, stream);
+        if (t.threads == 128 && t.registers == 56) return launch_variant<128, 9, 0>(s, a, counter, t, stream);
+        if (t.threads == 128 && t.registers == 48) return launch_variant<128, 10, 0>(s, a, counter, t, stream);
+        if (t.threads == 128 && t.registers == 80) return launch_variant<128, 6, 0>(s, a, counter, t, stream);
+        if (t.threads == 256 && t.registers == 64) return launch_variant<256, 4, 0>(s, a, counter, t, stream);
         return cudaErrorInvalidValue;
     }
     const bool small = s.per_world <= 32;
     if (t.threads == 128 && t.registers == 64)
-        return small ? launch_variant<128, 8, 32>(s, a, counter, t, stream, after_camera, after_shade)
-                     : launch_variant<128, 8, TILE_MAX_INSTANCES>(s, a, counter, t, stream, after_camera, after_shade);
+        return small ? launch_variant<128, 8, 32>(s, a, counter, t, stream)
+                     : launch_variant<128, 8, TILE_MAX_INSTANCES>(s, a, counter, t, stream);
     if (t.threads == 128 && t.registers == 56)
-        return small ? launch_variant<128, 9, 32>(s, a, counter, t, stream, after_camera, after_shade)
-                     : launch_variant<128, 9, TILE_MAX_INSTANCES>(s, a, counter, t, stream, after_camera, after_shade);
+        return small ? launch_variant<128, 9, 32>(s, a, counter, t, stream)
+                     : launch_variant<128, 9, TILE_MAX_INSTANCES>(s, a, counter, t, stream);
     if (t.threads == 128 && t.registers == 48)
-        return small ? launch_variant<128, 10, 32>(s, a, counter, t, stream, after_camera, after_shade)
-                     : launch_variant<128, 10, TILE_MAX_INSTANCES>(s, a, counter, t, stream, after_camera, after_shade);
+        return small ? launch_variant<128, 10, 32>(s, a, counter, t, stream)
+                     : launch_variant<128, 10, TILE_MAX_INSTANCES>(s, a, counter, t, stream);
     if (t.threads == 128 && t.registers == 80)
-        return small ? launch_variant<128, 6, 32>(s, a, counter, t, stream, after_camera, after_shade)
-                     : launch_variant<128, 6, TILE_MAX_INSTANCES>(s, a, counter, t, stream, after_camera, after_shade);
+        return small ? launch_variant<128, 6, 32>(s, a, counter, t, stream)
+                     : launch_variant<128, 6, TILE_MAX_INSTANCES>(s, a, counter, t, stream);
     if (t.threads == 256 && t.registers == 64)
-        return small ? launch_variant<256, 4, 32>(s, a, counter, t, stream, after_camera, after_shade)
-                     : launch_variant<256, 4, TILE_MAX_INSTANCES>(s, a, counter, t, stream, after_camera, after_shade);
+        return small ? launch_variant<256, 4, 32>(s, a, counter, t, stream)
+                     : launch_variant<256, 4, TILE_MAX_INSTANCES>(s, a, counter, t, stream);
     return cudaErrorInvalidValue;
 }
 
