@@ -12,6 +12,8 @@
 // group cannot finish are the inter-world ones (never traversed: every ray starts at its world's root);
 // their links are emitted by the group that owns their index, and a second small launch fits their boxes
 // by climbing from the world roots, as fit_boxes does (cuda_tlas.cuh:179-196).
+#include <climits>
+
 #include "device.cuh"
 #include "kernels.h"
 
@@ -115,31 +117,80 @@ struct GroupSmem {
     int bounds[6];         // ordered-int centre bounds
 };
 
-// The reference's common_prefix (cuda_tlas.cuh:119-124) between sorted positions p (in this world) and x,
-// from this world's keys in shared memory and, for a position in another world, from the world numbers
-// alone: keys of different worlds first differ in the world bits, so their shared prefix is clz32(w ^ wx).
+// A node of the radix tree over all worlds' sorted keys (build_radix_tree, cuda_tlas.cuh:128-159): its range's two ends and
+// the last position of its left part, as sorted positions.
+struct RadixNode {
+    int lo, hi, gamma;
+};
+
+// The node at local position i of a world of P instances whose range lies inside the world (0 < i < P - 1, or the world's
+// root from one of its ends): the reference's searches over the world's keys in shared memory, where common_prefix
+// (cuda_tlas.cuh:119-124) is 32 world bits and the Morton codes' shared bits, equal keys told apart by their positions.
+// A position outside the world shares fewer than the 32 world bits, which no node of these reaches: -1.
 template <int G>
-__device__ __forceinline__ int delta(const GroupSmem<G> &sm, int p, long long x, long long n, long long base, int P,
-    uint32_t world, uint32_t key_p, const int *world_first, int worlds) {
-    if (x < 0 || x >= n) return -1;
-    if (x >= base && x < base + P) {
-        const uint32_t kx = sm.key[x - base];
-        if (kx == key_p) return 64 + __clz(static_cast<int>(static_cast<uint32_t>(p) ^ static_cast<uint32_t>(x)));
-        return 32 + __clz(static_cast<int>(key_p ^ kx));
+__device__ __forceinline__ RadixNode node_inside(const GroupSmem<G> &sm, int i, int P, int base) {
+    const uint32_t kp = sm.key[i];
+    auto prefix = [&](int x) -> int {
+        if (static_cast<unsigned>(x) >= static_cast<unsigned>(P)) return -1;
+        const uint32_t kx = sm.key[x];
+        return kx == kp ? 64 + __clz((base + i) ^ (base + x)) : 32 + __clz(static_cast<int>(kp ^ kx));
+    };
+    const int d = prefix(i + 1) > prefix(i - 1) ? 1 : -1;
+    const int min_prefix = prefix(i - d);
+    int max_length = 2;
+    while (prefix(i + max_length * d) > min_prefix) max_length *= 2;
+    int length = 0;
+    for (int t = max_length / 2; t >= 1; t /= 2)
+        if (prefix(i + (length + t) * d) > min_prefix) length += t;
+    const int j = i + length * d;
+    const int node_prefix = prefix(j);
+    int s = 0;
+    for (int t = (length + 1) / 2;; t = (t + 1) / 2) {
+        if (prefix(i + (s + t) * d) > node_prefix) s += t;
+        if (t == 1) break;
     }
-    uint32_t wx;
-    if (world_first) {  // uneven worlds: the last world whose first instance is at most x
-        int lo = 0, hi = worlds - 1;
+    const int gamma = i + s * d + (d < 0 ? d : 0);
+    return RadixNode{base + min(i, j), base + max(i, j), base + gamma};
+}
+
+// The node at a world's first or last position (global position p), whose range goes on over other worlds or is the
+// world itself (then `inside`). Keys of different worlds first differ in their world numbers, so the worlds that share
+// more than k bits with world w are those of an aligned block of numbers, and the reference's searches end at the
+// blocks' ends: no search.
+struct WorldRuns {
+    const int *first;  // uneven worlds: each world's first instance (and the total past the last), or null
+    int per_world, worlds, n;
+    __device__ __forceinline__ int begin(int w) const { return first ? __ldg(first + w) : w * per_world; }
+    __device__ __forceinline__ int world_of(int x) const {
+        if (!first) return x / per_world;
+        int lo = 0, hi = worlds - 1;  // the last world whose first instance is at most x
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(world_first + mid) <= x) lo = mid;
+            if (__ldg(first + mid) <= x) lo = mid;
             else hi = mid - 1;
         }
-        wx = static_cast<uint32_t>(lo);
-    } else {
-        wx = static_cast<uint32_t>(x / P);
+        return lo;
     }
-    return __clz(static_cast<int>(world ^ wx));
+    // Bits that the key at x shares with world w's (x in another world), -1 past the ends.
+    __device__ __forceinline__ int prefix(int w, int x) const {
+        return x < 0 || x >= n ? -1 : __clz(w ^ world_of(x));
+    }
+    // The last position (d > 0) or the first (d < 0) of the worlds that share more than k bits with world w.
+    __device__ __forceinline__ int block_end(int w, int k, int d) const {
+        const unsigned low = k < 0 ? 0xffffffffu : 0x7fffffffu >> k;  // the bits past the first k + 1
+        if (d < 0) return begin(static_cast<int>(static_cast<unsigned>(w) & ~low));
+        const unsigned last = static_cast<unsigned>(w) | low;
+        return (last >= static_cast<unsigned>(worlds) ? n : begin(static_cast<int>(last) + 1)) - 1;
+    }
+};
+__device__ __forceinline__ RadixNode node_at_world_end(const WorldRuns &runs, int w, int p, int base, int P, bool &inside) {
+    // Towards the side that shares more: into the world, unless it is this one instance.
+    const int d = P > 1 ? (p == base ? 1 : -1) : runs.prefix(w, p + 1) > runs.prefix(w, p - 1) ? 1 : -1;
+    const int j = runs.block_end(w, runs.prefix(w, p - d), d);
+    const int wj = runs.world_of(j);
+    inside = wj == w;
+    const int split = inside ? 0 : runs.block_end(w, __clz(w ^ wj), d);  // the last position on p's side
+    return RadixNode{min(p, j), max(p, j), d > 0 ? split : split - 1};
 }
 
 // World w's climb from its root through the inter-world nodes: the second arrival at a node computes its box from its
@@ -170,9 +221,44 @@ __device__ __forceinline__ void fit_world(int w, const int *roots, const int *pa
     }
 }
 
-// Few enough worlds for the build's last CTA to fit the inter-world nodes itself: up to four climbs a thread, against a
-// launch of its own (16 worlds, set and render: 118 -> 110 us without that launch, of which the climbs take back 4).
-__host__ __device__ constexpr int worlds_fit_inside(int threads) { return 4 * threads; }
+// The inter-world nodes' boxes by one CTA, for at most a world per thread: the worlds' root boxes in shared memory, and each
+// node's box from those of the worlds that its range covers. (A climb's level takes about 1.2 us of fences, atomics and
+// dependent loads, and 16 worlds take four; here no thread waits for another's node.)
+__device__ __forceinline__ void fit_worlds_inside(const BuildArgs &a, float *boxes, int threads) {
+    const int w = threadIdx.x, n = static_cast<int>(a.n);
+    if (w < a.worlds) {
+        const int root = __ldcg(a.roots + w);
+        float4 lo = make_float4(1e30f, 1e30f, 1e30f, 0.0f), hi = make_float4(-1e30f, -1e30f, -1e30f, 0.0f);
+        if (root >= 0) {
+            lo = __ldcg(a.tlas + 2LL * root);
+            hi = __ldcg(a.tlas + 2LL * root + 1);
+        }
+        const float b[6] = {lo.x, lo.y, lo.z, hi.x, hi.y, hi.z};
+        for (int k = 0; k < 6; ++k) boxes[k * threads + w] = b[k];
+    }
+    __syncthreads();
+    if (w >= a.worlds) return;
+    const WorldRuns runs{a.world_first, a.per_world, a.worlds, n};
+    const int base = runs.begin(w), P = runs.begin(w + 1) - base;
+    for (int e = 0; e < (P < 2 ? P : 2); ++e) {
+        const int p = e == 0 ? base : base + P - 1;
+        if (p >= n - 1) continue;
+        bool inside;
+        const RadixNode node = node_at_world_end(runs, w, p, base, P, inside);
+        if (inside) continue;
+        float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
+        for (int k = runs.world_of(node.lo), last = runs.world_of(node.hi); k <= last; ++k)
+            for (int c = 0; c < 3; ++c) {
+                lo[c] = fminf(lo[c], boxes[c * threads + k]);
+                hi[c] = fmaxf(hi[c], boxes[(3 + c) * threads + k]);
+            }
+        float *nd = reinterpret_cast<float *>(a.tlas + 2LL * p);  // its links are written
+        for (int c = 0; c < 3; ++c) {
+            nd[c] = lo[c];
+            nd[4 + c] = hi[c];
+        }
+    }
+}
 
 template <int G>
 __global__ void __launch_bounds__(G < 128 ? 128 : G) build_worlds_kernel(const BuildArgs a) {
@@ -234,10 +320,15 @@ __global__ void __launch_bounds__(G < 128 ? 128 : G) build_worlds_kernel(const B
                 hi[ax] = fmaxf(hi[ax], v);
             }
         }
-        for (int ax = 0; ax < 3; ++ax) {
-            const int c = to_ordered(0.5f * (lo[ax] + hi[ax]));
-            atomicMin(&sm.bounds[ax], c);
-            atomicMax(&sm.bounds[3 + ax], c);
+    }
+    // The world's centre bounds: a group is whole warps, so one atomic per warp and bound.
+    for (int ax = 0; ax < 3; ++ax) {
+        const int c = to_ordered(0.5f * (lo[ax] + hi[ax]));
+        const int mn = __reduce_min_sync(0xffffffffu, valid ? c : INT_MAX);
+        const int mx = __reduce_max_sync(0xffffffffu, valid ? c : INT_MIN);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&sm.bounds[ax], mn);
+            atomicMax(&sm.bounds[3 + ax], mx);
         }
     }
     if (world_ok && P == 0 && i == 0) a.roots[w] = -1;  // a world without instances has no tree
@@ -283,33 +374,25 @@ __global__ void __launch_bounds__(G < 128 ? 128 : G) build_worlds_kernel(const B
     }
     __syncthreads();
 
-    // The internal node at sorted position p = base + i (build_radix_tree, cuda_tlas.cuh:128-159).
+    // The internal node at sorted position p = base + i (build_radix_tree, cuda_tlas.cuh:128-159). Only a world's first
+    // and last can reach other worlds. (Searching all positions' keys, with the world of each one outside found by a
+    // division or a search, was most of the build: 24,000 cycles of a CTA's 40,000 at 120 instances a world, 70,000 of
+    // 95,000 in uneven worlds of up to 200; now 5,000 and 8,000.)
     const long long p = base + i;
     bool within = false, is_root = false;
     int left = 0, right = 0;
     if (valid && p < n - 1) {
-        const uint32_t kp = sm.key[i];
-        const uint32_t wu = static_cast<uint32_t>(w);
-        const int ip = static_cast<int>(p);
-        auto dlt = [&](long long x) { return delta<G>(sm, ip, x, n, base, P, wu, kp, a.world_first, a.worlds); };
-        const int d = dlt(p + 1) > dlt(p - 1) ? 1 : -1;
-        const int min_prefix = dlt(p - d);
-        long long max_length = 2;
-        while (dlt(p + max_length * d) > min_prefix) max_length *= 2;
-        long long length = 0;
-        for (long long t = max_length / 2; t >= 1; t /= 2)
-            if (dlt(p + (length + t) * d) > min_prefix) length += t;
-        const long long j = p + length * d;
-        const int node_prefix = dlt(j);
-        long long s = 0;
-        for (long long t = (length + 1) / 2;; t = (t + 1) / 2) {
-            if (dlt(p + (s + t) * d) > node_prefix) s += t;
-            if (t == 1) break;
+        const int ip = static_cast<int>(p), b = static_cast<int>(base), in = static_cast<int>(n);
+        RadixNode node{};
+        bool inside = true;
+        if (i == 0 || i == P - 1) {
+            const WorldRuns runs{a.world_first, a.per_world, a.worlds, in};
+            node = node_at_world_end(runs, static_cast<int>(w), ip, b, P, inside);
         }
-        const long long gamma = p + s * d + (d < 0 ? d : 0);
-        const long long rlo = p < j ? p : j, rhi = p < j ? j : p;
-        left = static_cast<int>((rlo == gamma) ? n - 1 + gamma : gamma);
-        right = static_cast<int>((rhi == gamma + 1) ? n - 1 + gamma + 1 : gamma + 1);
+        if (inside) node = node_inside<G>(sm, i, P, b);
+        const long long rlo = node.lo, rhi = node.hi;
+        left = node.lo == node.gamma ? in - 1 + node.gamma : node.gamma;
+        right = node.hi == node.gamma + 1 ? in - 1 + node.gamma + 1 : node.gamma + 1;
         a.parent[left] = ip;
         a.parent[right] = ip;
         within = rlo >= base && rhi <= base + P - 1;
@@ -377,8 +460,9 @@ __global__ void __launch_bounds__(G < 128 ? 128 : G) build_worlds_kernel(const B
         }
     }
 
-    // The last CTA to come here has every other's nodes before it.
-    if (a.built == nullptr || a.worlds < 2 || a.worlds > worlds_fit_inside(CTA)) return;
+    // The last CTA to come here has every other's nodes before it. (At most a world per thread: the build
+    // and the fit of 16 worlds 23 -> 12 us, one launch for two.)
+    if (a.built == nullptr || a.worlds < 2 || a.worlds > CTA) return;
     __shared__ int last;
     __threadfence();
     __syncthreads();
@@ -389,7 +473,7 @@ __global__ void __launch_bounds__(G < 128 ? 128 : G) build_worlds_kernel(const B
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int k = threadIdx.x; k < a.worlds; k += CTA) fit_world(k, a.roots, a.parent, a.arrivals, a.tlas, a.error_flag);
+    fit_worlds_inside(a, reinterpret_cast<float *>(smem_raw), CTA);
 }
 
 // The boxes of the inter-world nodes: one thread per world climbs from its root (fit_world).
@@ -795,7 +879,7 @@ cudaError_t launch_build_worlds(const BuildArgs &a, cudaStream_t stream) {
     }
     if (e != cudaSuccess) return e;
     const int threads = build_group_size(a.per_world) < 128 ? 128 : build_group_size(a.per_world);
-    if (a.worlds > 1 && (a.built == nullptr || a.worlds > worlds_fit_inside(threads))) {
+    if (a.worlds > 1 && (a.built == nullptr || a.worlds > threads)) {
         fit_world_links_kernel<<<(a.worlds + 127) / 128, 128, 0, stream>>>(a.roots, a.parent, a.arrivals, a.tlas,
             a.worlds, a.error_flag);
         e = cudaGetLastError();
