@@ -171,6 +171,7 @@ struct Renderer {
     int ray_kernel = 0;                       // ray queries: 0 automatic, 1 per thread, 2 persistent, 3 packets
     PersistentTuning tuning{128, 28, 72, 16};
     PersistentTuning tile_tuning{128, 0, 56, 0};
+    bool tile_tuning_set = false;             // chosen by the caller
     // Ray queries: the persistent kernel's shape measured best for them (no leaf batching), unless the caller
     // chose the persistent kernel and its shape.
     PersistentTuning ray_tuning{256, 28, 64, 1};
@@ -1122,7 +1123,11 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
             a.ended = work_counter.p + counters - 1;
             a.time_id = ++times_count;
         }
-        CK(launch_render_tiles(params, a, work_counter.p, tile_tuning, stream));
+        // Packet walks spill at 56 registers (100,000 instances at 1280 x 720: 1.206 ms, 1.158 at 64); candidate lists do
+        // not, and more warps serve them better (4096 worlds: 5.19 against 5.21).
+        PersistentTuning shape = tile_tuning;
+        if (!tile_tuning_set && per_world > TILE_MAX_INSTANCES) shape.registers = 64;
+        CK(launch_render_tiles(params, a, work_counter.p, shape, stream));
         stages = by_kernels ? 3 : 1;
     } else if (persistent) {
         a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
@@ -1625,6 +1630,7 @@ int ngb_set_tuning(ngb_renderer *h, int32_t kernel, int32_t threads_per_block, i
             r.kernel_choice = kernel;
             r.tile_tuning.threads = threads_per_block;
             r.tile_tuning.registers = registers;
+            r.tile_tuning_set = true;
             return;
         }
         const bool built = (threads_per_block == 128 && (registers == 48 || registers == 64 || registers == 72)) ||

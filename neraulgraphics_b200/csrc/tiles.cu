@@ -46,12 +46,9 @@ struct WarpSmem {
     int leaf[CAP];           // the candidates' leaves, smallest entry bound first (the view's order)
     float bound[CAP];        // and their bounds
 };
-// CAP 0: worlds of any size, walked as a packet (packet_walk); the warp's stack of the world tree's nodes.
+// CAP 0: worlds of any size, walked as a packet (packet_walk), which needs none.
 template <>
-struct WarpSmem<0> {
-    int ref[TLAS_STACK];
-    int count[TLAS_STACK];
-};
+struct WarpSmem<0> {};
 
 __device__ __forceinline__ float warp_max(float v) { return from_ordered(__reduce_max_sync(FULL, to_ordered(v))); }
 __device__ __forceinline__ float warp_min(float v) { return from_ordered(__reduce_min_sync(FULL, to_ordered(v))); }
@@ -207,24 +204,25 @@ __device__ __forceinline__ void closest_meshes(const SceneParams &s, const WarpS
 
 // A world's tree walked by the whole warp together (a packet), for the camera rays of worlds too large for
 // candidate lists: every internal node that some lane's ray enters before its closest hit so far is visited
-// once for all lanes, from child-pair records, the child the lanes enter first (least entry distance over the
-// lanes) before the other; an instance whose box a lane's ray enters is walked by that lane (instance_walk_body).
+// once for all lanes, from child-pair records, the child that more lanes enter first
+// before the other; an instance whose box a lane's ray enters is walked by that lane (instance_walk_body).
 // Each lane gets the hit its own walk of the tree finds, up to which of two equally distant hits is kept (the
-// instance order differs from a single ray's). The stack lives in the warp's shared memory.
+// instance order differs from a single ray's). The stack lives in the lanes' registers.
 // ANY (shadow rays): a lane stops at its first hit closer than tmax (hit_inst set to that instance), and the
 // packet ends once every lane has stopped; the answer does not depend on the order. skip: an instance the lane
 // leaves out (-1: none).
 template <bool ANY>
-__device__ __forceinline__ void packet_walk(const SceneParams &s, WarpSmem<0> &sm, int lane, int world, bool active,
+__device__ __forceinline__ void packet_walk(const SceneParams &s, int lane, int world, bool active,
     float3 o, float3 d, float &tmax, int &hit_inst, int &hit_tri, float &hu, float &hv, int skip, int max_steps,
     int *err) {
     const int root = s.instance_count > 0 ? __ldg(s.roots + world) : -1;
     if (root < 0) return;
     const float3 inv = safe_inverse(d);
-    int ref = root, count = 0, sp = 0;
+    // The packet's stack, one entry a lane in two registers: a node, or ~(instance) for one met on the stack.
+    int st_lo = 0, st_hi = 0, sp = 0;
+    int ref = root;
     if (root >= s.tlas_internal) {  // a world of one instance: its leaf is the root, taken as an instance met on the stack
-        ref = ~__float_as_int(__ldg(s.tlas + 2 * root).w);
-        count = -1;
+        ref = __float_as_int(__ldg(s.tlas + 2 * root).w);
     } else {
         const float4 lo = __ldg(s.tlas + 2 * root), hi = __ldg(s.tlas + 2 * root + 1);
         if (!__any_sync(FULL, active && box_entry(lo, hi, o, inv, tmax) < NO_HIT)) return;
@@ -241,41 +239,40 @@ __device__ __forceinline__ void packet_walk(const SceneParams &s, WarpSmem<0> &s
         // lane, at one place below (so the walk is inlined).
         int meet = -1;
         bool enters = false;
-        if (count < 0) {
+        if (ref < 0) {
             // An instance met on the stack: its leaf box first (leaf k of the sorted leaves is node n - 1 + k).
-            const float4 *leaf = s.tlas + 2 * (static_cast<long long>(s.tlas_internal) + __ldg(s.leaf_of + ref));
-            meet = ref;
+            meet = ~ref;
+            const float4 *leaf = s.tlas + 2 * (static_cast<long long>(s.tlas_internal) + __ldg(s.leaf_of + meet));
             enters = active && box_entry(__ldg(leaf), __ldg(leaf + 1), o, inv, tmax) < NO_HIT;
         } else {
             const float4 *q = s.tlas_pairs + 4 * static_cast<long long>(ref);
             const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
-            const bool open = active;
-            const float dl = open ? box_entry(make_float4(q0.x, q0.y, q0.z, 0.0f), make_float4(q0.w, q1.x, q1.y, 0.0f), o,
-                inv, tmax) : NO_HIT;
-            const float dr = open ? box_entry(make_float4(q1.z, q1.w, q2.x, 0.0f), make_float4(q2.y, q2.z, q2.w, 0.0f), o,
-                inv, tmax) : NO_HIT;
-            const bool hl = __any_sync(FULL, dl < NO_HIT), hr = __any_sync(FULL, dr < NO_HIT);
-            if (hl || hr) {
-                const bool left_first = !hr || (hl && warp_min(dl) <= warp_min(dr));
-                const int near_ref = __float_as_int(left_first ? q3.x : q3.z);
-                const int near_count = __float_as_int(left_first ? q3.y : q3.w);
-                if (hl && hr) {
+            float dl = box_entry(make_float4(q0.x, q0.y, q0.z, 0.0f), make_float4(q0.w, q1.x, q1.y, 0.0f), o, inv, tmax);
+            float dr = box_entry(make_float4(q1.z, q1.w, q2.x, 0.0f), make_float4(q2.y, q2.z, q2.w, 0.0f), o, inv, tmax);
+            if (!active) dl = dr = NO_HIT;
+            const unsigned ml = __ballot_sync(FULL, dl < NO_HIT), mr = __ballot_sync(FULL, dr < NO_HIT);
+            if ((ml | mr) != 0) {
+                // The child that more of the rays enter first goes first.
+                const bool left_first = mr == 0 ||
+                    (ml != 0 && __popc(__ballot_sync(FULL, dl < dr)) >= __popc(__ballot_sync(FULL, dr < dl)));
+                const int l = __float_as_int(q3.y) < 0 ? ~__float_as_int(q3.x) : __float_as_int(q3.x);
+                const int r = __float_as_int(q3.w) < 0 ? ~__float_as_int(q3.z) : __float_as_int(q3.z);
+                const int near_ref = left_first ? l : r;
+                if (ml != 0 && mr != 0) {
                     if (sp >= TLAS_STACK) {
                         if (lane == 0) *err = 1;
                         return;
                     }
-                    if (lane == 0) {
-                        sm.ref[sp] = __float_as_int(left_first ? q3.z : q3.x);
-                        sm.count[sp] = __float_as_int(left_first ? q3.w : q3.y);
-                    }
+                    const int far_ref = left_first ? r : l;
+                    if (lane == sp) st_lo = far_ref;
+                    if (lane + 32 == sp) st_hi = far_ref;
                     ++sp;
                 }
-                if (near_count < 0) {
-                    meet = near_ref;
+                if (near_ref < 0) {
+                    meet = ~near_ref;
                     enters = (left_first ? dl : dr) < NO_HIT;
                 } else {
                     ref = near_ref;
-                    count = near_count;
                     pop = false;
                 }
             }
@@ -292,12 +289,9 @@ __device__ __forceinline__ void packet_walk(const SceneParams &s, WarpSmem<0> &s
             hit_inst = meet;
         }
         if (pop) {
-            __syncwarp();
             if (sp == 0) return;
             --sp;
-            ref = sm.ref[sp];
-            count = sm.count[sp];
-            __syncwarp();
+            ref = __shfl_sync(FULL, sp < 32 ? st_lo : st_hi, sp & 31);
         }
     }
 }
@@ -774,7 +768,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) camera_tiles_kernel(const
                     closest_meshes(s, sm, leaves, ncand, T.pixel, eye, d, tmax, hit_inst, hit_tri, hu, hv, max_steps,
                         a.error_flag);
                 } else {
-                    packet_walk<false>(s, sm, lane, T.world, T.pixel, eye, d, tmax, hit_inst, hit_tri, hu, hv, -1,
+                    packet_walk<false>(s, lane, T.world, T.pixel, eye, d, tmax, hit_inst, hit_tri, hu, hv, -1,
                         max_steps, a.error_flag);
                 }
                 if (!T.pixel) continue;
@@ -1130,8 +1124,6 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_tiles_kernel(const
 template <int THREADS, int MIN_BLOCKS, bool BITS>
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_packets_kernel(const __grid_constant__ SceneParams s,
     const RenderArgs a, int *counter, long long tiles, int tiles_x, int tiles_per_view, int fetch) {
-    __shared__ WarpSmem<0> warp_smem[THREADS / 32];
-    WarpSmem<0> &sm = warp_smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int max_steps = s.blas_node_count + 2;
     if (!BITS && a.times) mark_begin(&a.times->shadow);
@@ -1157,7 +1149,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_packets_kernel(con
             const int skip = self_code >= 0 && (self_code & 3) == 1 ? self_code >> 2 : -1;
             float tmax = o4.w, hu = 0.0f, hv = 0.0f;
             int hit_inst = -1, hit_tri = -1;
-            packet_walk<true>(s, sm, lane, T.world, pending, mk3(o4.x, o4.y, o4.z), mk3(d4.x, d4.y, d4.z), tmax,
+            packet_walk<true>(s, lane, T.world, pending, mk3(o4.x, o4.y, o4.z), mk3(d4.x, d4.y, d4.z), tmax,
                 hit_inst, hit_tri, hu, hv, skip, max_steps, a.error_flag);
             const bool blocked = hit_inst >= 0;
             if (BITS) {
@@ -1180,8 +1172,6 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_packets_kernel(con
 template <int THREADS, int MIN_BLOCKS>
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) ray_packets_kernel(const __grid_constant__ SceneParams s,
     const RayArgs r, int *counter, long long groups, int groups_per_world) {
-    __shared__ WarpSmem<0> warp_smem[THREADS / 32];
-    WarpSmem<0> &sm = warp_smem[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int max_steps = s.blas_node_count + 2;
     for (;;) {
@@ -1211,7 +1201,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) ray_packets_kernel(const 
         // rays in all directions: 0.245 against 0.35 ms as packets; a 720-beam scan 0.13 against 0.17 ms).
         const float3 middle = mk3(__shfl_sync(FULL, d.x, 16), __shfl_sync(FULL, d.y, 16), __shfl_sync(FULL, d.z, 16));
         if (__all_sync(FULL, !live || dot(d, middle) > 0.0f))
-            packet_walk<false>(s, sm, lane, world, live, o, d, tmax, hit_inst, hit_tri, hu, hv, -1, max_steps, r.error_flag);
+            packet_walk<false>(s, lane, world, live, o, d, tmax, hit_inst, hit_tri, hu, hv, -1, max_steps, r.error_flag);
         else if (live)
             lane_walk<false>(s, world, o, d, tmax, hit_inst, hit_tri, hu, hv, -1, max_steps, r.error_flag);
         if (!valid) continue;
