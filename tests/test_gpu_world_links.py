@@ -19,8 +19,8 @@ def placed(rng, shape):
     return np.array(flat, np.float32).reshape(shape + (3, 4))
 
 
-@pytest.mark.parametrize("worlds,instances", [(1, 2), (2, 1), (3, 1), (7, 1), (64, 1), (127, 1), (128, 1), (129, 1), (513, 1), (5, 2), (6, 3),
-                                              (33, 5), (128, 3), (129, 3), (9, 31), (4, 32), (5, 33), (3, 64), (17, 100),
+@pytest.mark.parametrize("worlds,instances", [(1, 2), (2, 1), (3, 1), (7, 1), (64, 1), (127, 1), (128, 1), (129, 1), (1024, 1), (2047, 2), (2049, 1), (5, 2), (6, 3),
+                                              (33, 5), (128, 3), (129, 3), (9, 31), (4, 32), (5, 33), (3, 64), (17, 100), (1500, 2),
                                               (3, 200), (2, 513)])
 def test_batched_trees_are_the_oracles(worlds, instances):
     rng = np.random.default_rng(worlds * 1000 + instances)
