@@ -346,7 +346,7 @@ def run_ours(args, rank, world, local_rank, dist):
         dist.barrier()
     views = d.view_count
     value = world * views * K / (total_ms / 1000.0)
-    # Per-kernel GPU times of the render, from the library's events between its launches (untimed renders).
+    # Per-kernel GPU times of the render, taken by the render's own kernels (untimed renders).
     stage = []
     for s in range(5):
         r.render(cams_dev, wl.fov, 1, **kw)
@@ -490,10 +490,10 @@ def run_ours(args, rank, world, local_rank, dist):
                                     "frac": round(b_img * value / 1e9 / peak, 5)},
                      "issue": issue_figures()},
         "cpu_baseline": cpu,
-        # Per step: the tree build (compose + per-world build, inter-world links) and the render: the camera-basis
-        # kernel, the per-view candidate order and the camera, shade and shadow kernels (tile path), or the
-        # camera-basis and one render kernel.
-        "gpu_launches": (2 + (5 if len(stage_ms) == 3 else 2)) * K,
+        # Per step: the tree build (compose + per-world build; the inter-world links, which up to 128 worlds' build
+        # makes itself) and the render: its start (camera bases, candidate orders) and the camera, shade and shadow
+        # kernels (tile path), or the camera-basis and one render kernel.
+        "gpu_launches": ((2 if d.world_count > 128 else 1) + (4 if len(stage_ms) == 3 else 2)) * K,
         "kernel_shape": None if tuned is None else {k: tuned[k] for k in ("kernel", "threads", "registers", "refill",
                                                                             "leaf_batch", "fetch", "paired", "ms")},
         # The renderers' own device arrays (scene, trees, per-pixel scratch; ngb_device_bytes), not the images.
@@ -799,7 +799,7 @@ def uneven_figures(dev, K, W, seed=0, buckets=False):
            "shape_timings_ms": {f"{t['threads']}/{t['registers']} fetch {t['fetch']} "
                                 f"{'paired' if t['paired'] else 'one kind'}": round(t["ms"], 4)
                                 for t in tuned["timings"]},
-           "graph_matches_eager": same, "gpu_launches_per_step": 7,
+           "graph_matches_eager": same, "gpu_launches_per_step": 6,
            "workload": f"uneven_worlds: {views} worlds, {int(first[-1])} instances, {r.pixel_count} pixels; six "
                        "meshes of 12 to 20480 triangles; one light, spp 1, RGB+depth+ID"}
     if not buckets:

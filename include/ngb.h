@@ -311,15 +311,16 @@ int ngb_set_stream(ngb_renderer *r, void *cuda_stream);
 /* synchronous 1: calls wait for their work, at most timeout_seconds (NGB_TIMEOUT after that).
  * synchronous 0: calls return once the work is queued. */
 int ngb_set_sync(ngb_renderer *r, int32_t synchronous, double timeout_seconds);
-/* How renders run. kernel: 0 automatic (the tile kernels where they apply: one sample per pixel, at most one
- * light, no material with reflectivity >= 1e-3; else the per-pixel kernel), 1 the per-pixel kernel,
- * 2 the persistent kernel where it applies, 3 the tile kernels where the persistent kernel applies (worlds of
- * at most 256 instances through per-tile candidate lists, larger ones walking their tree as a warp packet).
- * Ray queries (ngb_cast_rays), unless ngb_set_ray_kernel chose otherwise, take warp packets in worlds above 256
- * instances (kernel 0 or 3) and else the persistent kernel in a shape of their own (256/64, refill 28, no leaf
- * batching), unless kernel 2 is chosen, whose shape they then take, or kernel 1 (the per-thread ray kernel).
+/* How renders run. kernel: 0 automatic and 3: the tile kernels (worlds of at most 256 instances through per-tile
+ * candidate lists, larger ones walking their tree as a warp packet), in one pass for one sample per pixel, at most one
+ * light and no material with reflectivity >= 1e-3, else a pass per sample and light; the per-pixel kernel where the
+ * passes' scratch cannot be had (no memory, or a stream capture before any such render). 1: the per-pixel kernel.
+ * 2: the persistent kernel where it applies (what takes one pass), else the per-pixel kernel.
+ * Ray queries (ngb_cast_rays), unless ngb_set_ray_kernel chose otherwise, take warp packets (kernel 0 or 3), the
+ * persistent kernel in its shape (kernel 2), or the per-thread ray kernel (kernel 1).
  * With kernel 3 the call sets the tile kernel's shape: threads_per_block and registers as one of 128/48,
- * 128/56, 128/64, 128/80, 256/64 (default 128/56); refill_lanes and leaf_batch are not read.
+ * 128/56, 128/64, 128/80, 256/64 (default 128/56, 128/64 for worlds above 256 instances); refill_lanes and
+ * leaf_batch are not read.
  * Otherwise it sets the persistent kernel's shape: threads_per_block and registers (the register budget per
  * thread) as one of 128/48, 128/64, 128/72, 256/48, 256/64, 64/64, refill_lanes (1..32: a warp takes new
  * pixels once this many of its lanes are free) and leaf_batch (1..32: lanes at a leaf wait until this many do,
@@ -334,12 +335,11 @@ int ngb_set_tuning(ngb_renderer *r, int32_t kernel, int32_t threads_per_block, i
  * are the same bit for bit either way. No counterpart in the reference. */
 int ngb_set_tile_shape(ngb_renderer *r, int32_t tiles_per_fetch, int32_t paired);
 
-/* Which kernel answers ray queries (ngb_cast_rays): 0 automatic (warp packets for worlds above 256 instances, else
- * as ngb_set_tuning describes), 1 one thread per ray, 2 the persistent kernel (lanes refilled as their rays end),
- * 3 warp packets: 32 consecutive rays of a world per
- * warp walking the world's tree together, each lane entering only what its own ray enters (for rays of one
- * sensor in scan order, such as a LiDAR's beams). The same hits every way, up to which of two equally distant hits
- * is kept. No counterpart in the reference. */
+/* Which kernel answers ray queries (ngb_cast_rays): 0 automatic (as ngb_set_tuning describes), 1 one thread per
+ * ray, 2 the persistent kernel (lanes refilled as their rays end), 3 warp packets: 32 consecutive rays of a world per
+ * warp walking the world's tree together, each lane entering only what its own ray enters (rays of one sensor in scan
+ * order, such as a LiDAR's beams), or each lane walking for itself where the warp's rays look all ways. The same
+ * hits every way, up to which of two equally distant hits is kept. No counterpart in the reference. */
 int ngb_set_ray_kernel(ngb_renderer *r, int32_t kernel);
 
 /* How the instance trees are built. mode 0 (default): one fused launch of per-world groups when a world

@@ -181,10 +181,12 @@ cudaError_t launch_rays_packets(const SceneParams &s, const RayArgs &r, int *cou
 // The tile render (see tiles.cu). Of the tuning, threads and registers are read: 128/48, 128/56, 128/64, 128/80 or
 // 256/64. counters: tile_counters(a, lights) zeroed counters, one for each launch that takes tiles from a queue.
 constexpr int TILE_MAX_INSTANCES = 256;  // the largest world rendered from candidate lists
+constexpr int TILE_COUNTERS = 3 + MAX_LIGHTS;
 inline bool one_pass(const RenderArgs &a, int lights) { return a.spp == 1 && lights <= 1 && !a.reflective; }
 inline size_t tile_counters(const RenderArgs &a, int lights) {
-    // One more counts the ended warps of the last kernel of a render that is timed by its kernels.
-    return 1 + (!a.rgb ? 1 : one_pass(a, lights) ? 2 : static_cast<size_t>(a.spp) * (2 + lights));
+    // One more counts the ended warps of the last kernel of a render that is timed by its kernels; a sample of several
+    // starts them again, so that no render needs more than TILE_COUNTERS (a captured graph holds their address).
+    return 1 + (!a.rgb ? 1 : one_pass(a, lights) ? 2 : 2 + static_cast<size_t>(lights));
 }
 cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, unsigned long long *counters, const PersistentTuning &t,
     cudaStream_t stream);

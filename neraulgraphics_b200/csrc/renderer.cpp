@@ -379,7 +379,7 @@ void Renderer::init(const ngb_scene &s, const UnevenLayout *layout) {
     for (int i = 0; i < s.sphere_count; ++i) reflective = reflective || s.spheres[i].material.reflectivity >= 1e-3f;
     reflective = reflective || (s.floor.half_extent_x > 0.0f && s.floor.material.reflectivity >= 1e-3f);
     for (int i = 0; i < s.instance_count; ++i) reflective = reflective || s.instances[i].material.reflectivity >= 1e-3f;
-    work_counter.ensure(1);
+    work_counter.ensure(TILE_COUNTERS);
     {
         float table[256];
         srgb_thresholds(table);
@@ -994,7 +994,7 @@ bool Renderer::pass_scratch(const RenderArgs &a, int views, bool single) {
         return true;
     };
     try {
-        bool ok = have(camera_basis, 3 * nv) && have(work_counter, tile_counters(a, params.light_count));
+        bool ok = have(camera_basis, 3 * nv);
         if (per_world > 0 && per_world <= TILE_MAX_INSTANCES)
             ok = ok && have(view_order, nv * per_world) && have(view_bound, nv * per_world);
         if (a.rgb)
@@ -1116,7 +1116,6 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
             a.visible = sample_visible.ensure(pixels());
         }
         const size_t counters = tile_counters(a, params.light_count);
-        work_counter.ensure(counters);
         if (by_kernels) {
             // The times of a render before this one that nobody read are given up: it writes the same place.
             a.times = times.p;

@@ -1,5 +1,6 @@
-// The tile render kernels: the batched path's common case (one sample per pixel, at most one light, no mirror
-// bounces), in three launches (camera rays, shading, shadow rays), for worlds of any size: candidate lists for
+// The tile render kernels: the batched path, its common case (one sample per pixel, at most one light, no mirror
+// bounces) in four launches (setup, camera rays, shading, shadow rays) and pictures of several samples, lights or
+// mirrors in passes of them (sample passes, below), for worlds of any size: candidate lists for
 // worlds of up to TILE_MAX_INSTANCES instances (what a batch of simulator worlds holds), a packet walk of the
 // world tree above that.
 //
@@ -1565,6 +1566,9 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, unsigned l
         unsigned long long *counter = counters;
         for (b.sample = 0; b.sample < a.spp && e == cudaSuccess; ++b.sample) {
             if (b.sample > 0) {
+                counter = counters;
+                e = cudaMemsetAsync(counters, 0, tile_counters(a, s.light_count) * sizeof(unsigned long long), stream);
+                if (e != cudaSuccess) return e;
                 b.rng_in = a.rng_out;
                 b.depth = b.normal = nullptr;
                 b.object_id = b.hit_instance = nullptr;
@@ -1588,7 +1592,6 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, unsigned l
                 if (groups > static_cast<long long>(PER_SM) * sms) groups = static_cast<long long>(PER_SM) * sms;
                 bounce_kernel<THREADS_B, PER_SM><<<static_cast<unsigned>(groups), THREADS_B, 0, stream>>>(s, b);
             }
-            ++counter;
             e = cudaGetLastError();
         }
         return e;

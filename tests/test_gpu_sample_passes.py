@@ -83,3 +83,21 @@ def test_a_capture_without_a_render_before_it_takes_the_kernel_that_needs_no_scr
     want = images(r, cams, 0, 2, rgb=True)["rgb"]
     differ = (into["rgb"].cpu().numpy() != want).any(-1).sum()
     assert differ <= 2 * 32 * 32 * 1e-3
+
+
+def test_a_captured_render_outlives_renders_of_more_samples():
+    import torch
+    r, cams = scene(2, 6, 2, True, 32, 32)
+    dev = torch.from_numpy(cams).cuda()
+    into = {"rgb": torch.zeros((2, 32, 32, 3), dtype=torch.uint8, device="cuda")}
+    r.render(dev, 1.0, 2, frame=3, rgb=True, into=into)
+    torch.cuda.synchronize()
+    want = into["rgb"].clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        r.render(dev, 1.0, 2, frame=3, rgb=True, into=into)
+    r.render(dev, 1.0, 9, frame=1, rgb=True, into=into)
+    into["rgb"].zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(into["rgb"], want)
