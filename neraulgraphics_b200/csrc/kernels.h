@@ -129,7 +129,8 @@ struct RenderArgs {
     // The render's GPU times, taken by its kernels (null: not timed): when it, its shading and its shadow rays began and
     // when its last kernel's last warp ended.
     RenderTimes *times;
-    unsigned long long *ended;     // zeroed: the warps of the last kernel that have ended
+    unsigned long long *ended;     // zeroed: the warps of the last kernel that have ended; null when that is not one of the
+                                   // camera or shadow kernels (launch_mark_end then marks the end)
     unsigned long long time_id;    // what the last warp leaves in times->id
 };
 
@@ -190,6 +191,8 @@ inline size_t tile_counters(const RenderArgs &a, int lights) {
 }
 cudaError_t launch_render_tiles(const SceneParams &s, const RenderArgs &a, unsigned long long *counters, const PersistentTuning &t,
     cudaStream_t stream);
+// The end of a timed render (a.ended set), in a launch of its own after its last kernel.
+cudaError_t launch_mark_end(const RenderArgs &a, cudaStream_t stream);
 
 // The adjoint of the depth and normal images (see adjoint.cu). Every pointer is device memory; grad_normal
 // may be null; the gradients are added to grad_matrices and grad_cameras.

@@ -1086,8 +1086,8 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         "reflective material");
     // Inside a CUDA graph capture the timing events would be graph nodes whose times cannot be read: the
     // render is then not timed (last_kernel_ms keeps the previous figure).
-    const bool timed = !capturing(), by_kernels = timed && tiles && single && !a.radiance && pixels() > 0 &&
-        (!a.rgb || params.light_count == 1);
+    const bool timed = !capturing(), by_kernels = timed && tiles && single && pixels() > 0;
+    unsigned long long *ended = nullptr;
     if (timed && !by_kernels) CK(cudaEventRecord(ev_start, stream));
     if (tiles) {
         a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
@@ -1119,7 +1119,8 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         if (by_kernels) {
             // The times of a render before this one that nobody read are given up: it writes the same place.
             a.times = times.p;
-            a.ended = work_counter.p + counters - 1;
+            ended = work_counter.p + counters - 1;
+            if (!a.radiance && (!a.rgb || params.light_count == 1)) a.ended = ended;
             a.time_id = ++times_count;
         }
         // Packet walks spill at 56 registers (100,000 instances at 1280 x 720: 1.206 ms, 1.158 at 64); candidate lists do
@@ -1139,6 +1140,10 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
     if (a.radiance)
         CK(launch_accumulate(a.radiance, view_accum.p, frame, static_cast<long long>(pixels()), srgb_table.p,
             view_argb.p, a.rgb, stream));
+    if (by_kernels && !a.ended) {
+        a.ended = ended;
+        CK(launch_mark_end(a, stream));
+    }
     if (timed) {
         times_id = by_kernels ? a.time_id : 0;
         if (!by_kernels) CK(cudaEventRecord(ev_stop, stream));

@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) camera_tiles_kernel(const
     for (;;) {
         const long long first = fetch_tiles(counter, lane, fetch);
         if (first >= tiles) {
-            if (!LATER && a.times && !a.rgb) mark_end(a);
+            if (!LATER && a.ended && !a.rgb) mark_end(a);
             break;
         }
         const long long last = first + fetch < tiles ? first + fetch : tiles;
@@ -1008,7 +1008,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_tiles_kernel(const
     for (;;) {
         const long long first = fetch_tiles(counter, lane, fetch);
         if (first >= tiles) {
-            if (!BITS && a.times) mark_end(a);
+            if (!BITS && a.ended) mark_end(a);
             break;
         }
         const long long last = first + fetch < tiles ? first + fetch : tiles;
@@ -1131,7 +1131,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) shadow_packets_kernel(con
     for (;;) {
         const long long first = fetch_tiles(counter, lane, fetch);
         if (first >= tiles) {
-            if (!BITS && a.times) mark_end(a);
+            if (!BITS && a.ended) mark_end(a);
             break;
         }
         const long long last = first + fetch < tiles ? first + fetch : tiles;
@@ -1606,6 +1606,15 @@ cudaError_t launch_variant(const SceneParams &s, const RenderArgs &a, unsigned l
 }
 
 }  // namespace
+
+namespace {
+__global__ void mark_end_kernel(const RenderArgs a) { mark_end(a); }
+}  // namespace
+
+cudaError_t launch_mark_end(const RenderArgs &a, cudaStream_t stream) {
+    mark_end_kernel<<<1, 32, 0, stream>>>(a);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_rays_packets(const SceneParams &s, const RayArgs &r, int *counter, cudaStream_t stream) {
     if (r.count <= 0 || r.rays_per_world <= 0) return cudaSuccess;

@@ -101,3 +101,13 @@ def test_a_captured_render_outlives_renders_of_more_samples():
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(into["rgb"], want)
+
+
+@pytest.mark.parametrize("lights,rgb", [(1, True), (0, True), (1, False)])
+def test_stage_times_of_one_pass(lights, rgb):
+    r, cams = scene(4, 8, lights, False, 64, 64)
+    for _ in range(2):
+        r.render(cams, 1.0, 1, rgb=rgb, depth=True)
+        stages = r.last_stage_ms
+        assert len(stages) == 3 and stages[0] > 0.0 and (stages[1] > 0.0) == rgb and (stages[2] > 0.0) == (rgb and lights == 1)
+        assert abs(sum(stages) - r.last_kernel_ms) <= 1e-5 and r.last_kernel_ms < 50.0
