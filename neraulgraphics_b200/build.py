@@ -2,8 +2,8 @@
 
     python -m neraulgraphics_b200.build
 
-Every kernel file but the adjoint is compiled with -fmad=false and IEEE division and square root: the arithmetic
-rules the kernels rely on for bit-exact parity (see csrc/device.cuh). The CUDA runtime is linked statically, so the
+Every kernel file is compiled with -fmad=false and IEEE division and square root: the arithmetic rules the
+kernels rely on for bit-exact parity (see csrc/device.cuh). The CUDA runtime is linked statically, so the
 library needs only the driver.
 """
 
@@ -21,7 +21,6 @@ OBJ = os.path.join(HERE, "_build")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CUDA_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
-CONTRACTED = ("adjoint.cu",)  # gradients: multiply-adds contracted
 SOURCES = ["lbvh.cu", "trace.cu", "persistent.cu", "tiles.cu", "adjoint.cu", "noalloc.cu", "blas_build.cu", "pose.cu", "host.cpp", "renderer.cpp"]
 
 
@@ -51,8 +50,7 @@ def build(verbose: bool = False) -> str:
         if not _stale(obj, [path] + headers):
             continue
         if src.endswith(".cu") or src == "renderer.cpp":
-            flags = ["-fmad=true" if f == "-fmad=false" and src in CONTRACTED else f for f in CUDA_FLAGS]
-            cmd = [nvcc(), "-x", "cu"] + ARCH + flags + ["-c", path, "-o", obj]
+            cmd = [nvcc(), "-x", "cu"] + ARCH + CUDA_FLAGS + ["-c", path, "-o", obj]
         else:
             cmd = [nvcc(), "-std=c++17", "-O3", "-Xcompiler", "-fPIC,-Wall", "-c", path, "-o", obj]
         res = subprocess.run(cmd, capture_output=True, text=True)

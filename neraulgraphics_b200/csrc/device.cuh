@@ -1,6 +1,6 @@
 // Device-side types and math shared by the kernels (compose + tree build, trace, ray queries).
 //
-// Arithmetic rules. Every kernel file but the adjoint's is compiled with -fmad=false and IEEE division and square root, and
+// Arithmetic rules. Every kernel file is compiled with -fmad=false and IEEE division and square root, and
 // every expression keeps the reference's operation order (src/geom_dev.h, src/render_core.h,
 // src/mesh_dev.h, src/cuda_tlas.cuh), so a hit, a depth or a normal is bit-for-bit what the reference's
 // CPU backend computes from the same inputs. normalize is v * (1 / sqrt(v.v)) as the reference's host
