@@ -156,9 +156,23 @@ struct Renderer {
     DevBuf<float4> camera_basis;              // the persistent and tile renders' per-view cameras
     DevBuf<float4> pic_hit, shadow_o, shadow_d;  // the tile render's per-pixel hand-over between its kernels
     DevBuf<int> pic_code, shadow_self;
-    DevBuf<uint32_t> sample_rng;              // between the samples of a picture (tiles.cu, sample passes)
-    DevBuf<float4> sample_sum;
-    DevBuf<uint8_t> sample_visible;
+    // What the tile kernels need for the renders that the per-pixel kernel could do without any of it (several samples,
+    // lights or mirrors: tiles.cu, sample passes). A set of its own, and each such render waits for the one before it on
+    // whatever stream that ran (`done`), so renders on several streams, replayed captures among them, stay independent
+    // of each other and of the renders above.
+    struct PassScratch {
+        DevBuf<float4> basis, hit, shadow_o, shadow_d, sum;
+        DevBuf<int> code, self, order;
+        DevBuf<float> bound;
+        DevBuf<uint32_t> rng;
+        DevBuf<uint8_t> visible;
+        DevBuf<unsigned long long> counters;
+        cudaEvent_t done = nullptr;
+        void release() {
+            basis.release(), hit.release(), shadow_o.release(), shadow_d.release(), sum.release(), code.release();
+            self.release(), order.release(), bound.release(), rng.release(), visible.release(), counters.release();
+        }
+    } passes;
     DevBuf<int> view_order;                   // the tile render's per-view candidate order, and its bounds
     DevBuf<float> view_bound;
     DevBuf<float> srgb_table;                 // 256 sRGB byte thresholds
@@ -273,7 +287,7 @@ struct Renderer {
     void put_lights(const ngb_light *lights, int count);
     void cast_rays(const float *o, const float *d, int rays_per_world, float max_distance, int memory, ngb_ray_hits *out,
         float *distance, float *normal, int32_t *ids);
-    bool pass_scratch(const RenderArgs &a, int views, bool single);
+    bool pass_scratch(RenderArgs &a, int views, bool single);
     int rows() const { return band_rows > 0 ? band_rows : height; }
     size_t pixels() const {
         return uneven ? static_cast<size_t>(total_pixels) : static_cast<size_t>(worlds) * cpw * rows() * width;
@@ -361,6 +375,7 @@ void Renderer::init(const ngb_scene &s, const UnevenLayout *layout) {
     times.ensure(1);
     CK(cudaMemsetAsync(times.p, 0, sizeof(RenderTimes), stream));
     CK(cudaEventCreateWithFlags(&ev_done, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&passes.done, cudaEventDisableTiming));
     CK(cudaHostAlloc(&host_error, sizeof(int), cudaHostAllocDefault));
     CK(cudaHostAlloc(&host_count, sizeof(int), cudaHostAllocDefault));
     *host_error = 0;
@@ -562,12 +577,13 @@ void Renderer::teardown() {
     if (ev_start) cudaEventDestroy(ev_start);
     if (ev_stop) cudaEventDestroy(ev_stop);
     if (ev_done) cudaEventDestroy(ev_done);
+    if (passes.done) cudaEventDestroy(passes.done);
     if (host_error) cudaFreeHost(host_error);
     if (host_count) cudaFreeHost(host_count);
     if (host_times) cudaFreeHost(host_times);
     times.release();
     if (own_stream) cudaStreamDestroy(own_stream);
-    ev_start = ev_stop = ev_done = nullptr;
+    ev_start = ev_stop = ev_done = passes.done = nullptr;
     host_error = host_count = nullptr;
     host_times = nullptr;
     own_stream = nullptr;
@@ -586,7 +602,7 @@ void Renderer::teardown() {
     blas_pairs.release(), tlas_pairs.release(), slot_root.release(), work_counter.release();
     large_aabb.release(), large_bounds.release(), large_ids_a.release(), large_ids_b.release();
     large_keys_a.release(), large_keys_b.release(), large_counts.release();
-    sample_rng.release(), sample_sum.release(), sample_visible.release();
+    passes.release();
     pic_hit.release(), shadow_o.release(), shadow_d.release(), pic_code.release(), shadow_self.release();
     view_order.release(), view_bound.release();
     leaf_of.release(), slot_hull.release(), slot_sphere.release();
@@ -983,29 +999,47 @@ void Renderer::check_view(const ngb_camera *c, int frame, int spp) {
 }
 
 // The tile kernels' scratch for a render that the per-pixel kernel could do too: false where it cannot be had (no
-// memory left, not allocated yet when a capture forbids it, or more pixels than the passes' lists can name).
-bool Renderer::pass_scratch(const RenderArgs &a, int views, bool single) {
-    const size_t px = pixels(), nv = static_cast<size_t>(views);
-    if (px > static_cast<size_t>(INT32_MAX)) return false;
+// memory left, more pixels than the passes' lists can name, or a capture when it is not there for the whole image: a
+// graph keeps these addresses, and what holds every row of the image is never outgrown and so stays until the renderer
+// goes).
+bool Renderer::pass_scratch(RenderArgs &a, int views, bool single) {
     const bool fixed = capturing();
+    const size_t nv = static_cast<size_t>(views), px = fixed ? nv * height * width : pixels();
+    if (px > static_cast<size_t>(INT32_MAX)) return false;
     auto have = [&](auto &buf, size_t count) {
         if (fixed) return buf.n >= count;
         buf.ensure(count);
         return true;
     };
     try {
-        bool ok = have(camera_basis, 3 * nv);
+        bool ok = have(passes.basis, 3 * nv) && have(passes.counters, TILE_COUNTERS);
         if (per_world > 0 && per_world <= TILE_MAX_INSTANCES)
-            ok = ok && have(view_order, nv * per_world) && have(view_bound, nv * per_world);
+            ok = ok && have(passes.order, nv * per_world) && have(passes.bound, nv * per_world);
         if (a.rgb)
-            ok = ok && have(pic_hit, px) && have(pic_code, px) && have(shadow_o, px) && have(shadow_d, px) &&
-                have(shadow_self, px);
-        if (!single) ok = ok && have(sample_rng, px) && have(sample_sum, px) && have(sample_visible, px);
-        return ok;
+            ok = ok && have(passes.hit, px) && have(passes.code, px) && have(passes.shadow_o, px) &&
+                have(passes.shadow_d, px) && have(passes.self, px);
+        if (!single) ok = ok && have(passes.rng, px) && have(passes.sum, px) && have(passes.visible, px);
+        if (!ok) return false;
     } catch (const CudaFailure &) {
         cudaGetLastError();
         return false;
     }
+    if (!a.basis_given) a.camera_basis = passes.basis.p;
+    a.view_order = passes.order.p;
+    a.view_bound = passes.bound.p;
+    if (a.rgb) {
+        a.pic_hit = passes.hit.p;
+        a.pic_code = passes.code.p;
+        a.shadow_o = passes.shadow_o.p;
+        a.shadow_d = passes.shadow_d.p;
+        a.shadow_self = passes.self.p;
+    }
+    if (!single) {
+        a.rng_out = passes.rng.p;
+        a.sample_sum = passes.sum.p;
+        a.visible = passes.visible.p;
+    }
+    return true;
 }
 
 void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, int frame, int memory, uint8_t *rgb,
@@ -1073,6 +1107,7 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
     // The per-pixel kernel needs no scratch: pictures that the tile kernels take several passes for go to it where the
     // passes' scratch cannot be had.
     if (tiles && !persistent_ok) tiles = pass_scratch(a, views, single);
+    const bool in_passes = tiles && !persistent_ok;
     const bool persistent = !view && !tiles && persistent_ok && (kernel_choice == 0 || kernel_choice == 2);
     if (view && a.rgb) {
         a.radiance = view_radiance.ensure(pixels());
@@ -1086,34 +1121,31 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         "reflective material");
     // Inside a CUDA graph capture the timing events would be graph nodes whose times cannot be read: the
     // render is then not timed (last_kernel_ms keeps the previous figure).
-    const bool timed = !capturing(), by_kernels = timed && tiles && single && pixels() > 0;
+    const bool timed = !capturing(), by_kernels = timed && tiles && !in_passes && pixels() > 0;
     unsigned long long *ended = nullptr;
     if (timed && !by_kernels) CK(cudaEventRecord(ev_start, stream));
     if (tiles) {
-        a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
-        if (per_world > 0 && per_world <= TILE_MAX_INSTANCES) {
-            a.view_order = view_order.ensure(static_cast<size_t>(views) * per_world);
-            a.view_bound = view_bound.ensure(static_cast<size_t>(views) * per_world);
-            a.order_stride = per_world;
+        if (!in_passes) {
+            a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
+            if (per_world > 0 && per_world <= TILE_MAX_INSTANCES) {
+                a.view_order = view_order.ensure(static_cast<size_t>(views) * per_world);
+                a.view_bound = view_bound.ensure(static_cast<size_t>(views) * per_world);
+            }
+            if (a.rgb) {
+                a.pic_hit = pic_hit.ensure(pixels());
+                a.pic_code = pic_code.ensure(pixels());
+                a.shadow_o = shadow_o.ensure(pixels());
+                a.shadow_d = shadow_d.ensure(pixels());
+                a.shadow_self = shadow_self.ensure(pixels());
+            }
         }
+        if (per_world > 0 && per_world <= TILE_MAX_INSTANCES) a.order_stride = per_world;
         if (uneven) {
             a.view_info = view_info.p;
             a.total_pixels = total_pixels;
             a.total_tiles = total_tiles;
             a.view_pair_tile = view_pair_tile.p;
             a.total_pair_tiles = total_pair_tiles;
-        }
-        if (a.rgb) {
-            a.pic_hit = pic_hit.ensure(pixels());
-            a.pic_code = pic_code.ensure(pixels());
-            a.shadow_o = shadow_o.ensure(pixels());
-            a.shadow_d = shadow_d.ensure(pixels());
-            a.shadow_self = shadow_self.ensure(pixels());
-        }
-        if (!single) {
-            a.rng_out = sample_rng.ensure(pixels());
-            a.sample_sum = sample_sum.ensure(pixels());
-            a.visible = sample_visible.ensure(pixels());
         }
         const size_t counters = tile_counters(a, params.light_count);
         if (by_kernels) {
@@ -1127,7 +1159,10 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         // not, and more warps serve them better (4096 worlds: 5.19 against 5.21).
         PersistentTuning shape = tile_tuning;
         if (!tile_tuning_set && per_world > TILE_MAX_INSTANCES) shape.registers = 64;
-        CK(launch_render_tiles(params, a, work_counter.p, shape, stream));
+        // A capture waits for and marks the event each time it is replayed.
+        if (in_passes) CK(cudaStreamWaitEvent(stream, passes.done, timed ? 0 : cudaEventWaitExternal));
+        CK(launch_render_tiles(params, a, in_passes ? passes.counters.p : work_counter.p, shape, stream));
+        if (in_passes) CK(cudaEventRecordWithFlags(passes.done, stream, timed ? 0 : cudaEventRecordExternal));
         stages = by_kernels ? 3 : 1;
     } else if (persistent) {
         a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
