@@ -1432,13 +1432,15 @@ template <int THREADS, int MIN_BLOCKS>
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) bounce_kernel(const __grid_constant__ SceneParams s, const RenderArgs a) {
     const int lane = threadIdx.x & 31;
     const int max_steps = s.blas_node_count + 2;
-    const int n = *a.bounces, per_view = a.width * a.rows;
+    const unsigned n = static_cast<unsigned>(*a.bounces);
+    const int per_view = a.width * a.rows;
     const float3 zero = mk3(0.0f, 0.0f, 0.0f);
-    const int warps = gridDim.x * (THREADS / 32);
-    int width = 4;
+    const unsigned warps = gridDim.x * (THREADS / 32);
+    unsigned width = 4;
     while (width < 32 && width * warps < n) width *= 2;
-    if (lane >= width) return;
-    for (int at = (blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5)) * width + lane; at < n; at += warps * width) {
+    if (static_cast<unsigned>(lane) >= width) return;
+    // Unsigned: a list may hold up to 2^31 - 1 pixels, and the last step goes past them.
+    for (unsigned at = (blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5)) * width + lane; at < n; at += warps * width) {
         const int p = a.shadow_self[at];
         const float4 o4 = a.shadow_o[p], d4 = a.shadow_d[p], r4 = a.pic_hit[p];
         float3 o = xyz(o4), d = xyz(d4), radiance = xyz(r4);
