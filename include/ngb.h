@@ -314,7 +314,8 @@ int ngb_set_sync(ngb_renderer *r, int32_t synchronous, double timeout_seconds);
 /* How renders run. kernel: 0 automatic and 3: the tile kernels (worlds of at most 256 instances through per-tile
  * candidate lists, larger ones walking their tree as a warp packet), in one pass for one sample per pixel, at most one
  * light and no material with reflectivity >= 1e-3, else a pass per sample and light; the per-pixel kernel where the
- * passes' scratch cannot be had (no memory, or a stream capture before any such render). 1: the per-pixel kernel.
+ * passes' scratch (77 bytes per pixel, kept) cannot be had: no memory (not tried again for as many pixels until
+ * ngb_set_rows), or a stream capture before any such render of the whole image. 1: the per-pixel kernel.
  * 2: the persistent kernel where it applies (what takes one pass), else the per-pixel kernel.
  * Ray queries (ngb_cast_rays), unless ngb_set_ray_kernel chose otherwise, take warp packets (kernel 0 or 3), the
  * persistent kernel in its shape (kernel 2), or the per-thread ray kernel (kernel 1).
@@ -355,8 +356,9 @@ int64_t ngb_device_bytes(void);
  * one), fails as cudaMalloc does for lack of memory: the call that made it returns NGB_CUDA_ERROR ("out of
  * memory"). A renderer under construction is not made and frees all it made; a renderer stays usable (a failed
  * set_* call leaves the previous tree in place, a failed render leaves its outputs unwritten) and keeps the
- * arrays it made before the failure for its next call. after < 0 cancels. No GPU fault is involved. No
- * counterpart in the reference. */
+ * arrays it made before the failure for its next call. A render whose passes' scratch fails (ngb_set_tuning) is no
+ * error: the per-pixel kernel draws it and the scratch per pixel is freed. after < 0 cancels. No GPU fault is
+ * involved. No counterpart in the reference. */
 int ngb_inject_allocation_failure(int32_t after);
 
 /* The rows every later render draws: image rows [first, first + count) of every view, count >= 1 and

@@ -168,9 +168,14 @@ struct Renderer {
         DevBuf<uint8_t> visible;
         DevBuf<unsigned long long> counters;
         cudaEvent_t done = nullptr;
+        size_t refused = 0;  // pixels whose arrays could not be allocated (0: none)
+        void release_pixels() {
+            hit.release(), code.release(), shadow_o.release(), shadow_d.release(), self.release();
+            rng.release(), sum.release(), visible.release();
+        }
         void release() {
-            basis.release(), hit.release(), shadow_o.release(), shadow_d.release(), sum.release(), code.release();
-            self.release(), order.release(), bound.release(), rng.release(), visible.release(), counters.release();
+            release_pixels();
+            basis.release(), order.release(), bound.release(), counters.release();
         }
     } passes;
     DevBuf<int> view_order;                   // the tile render's per-view candidate order, and its bounds
@@ -1006,6 +1011,7 @@ bool Renderer::pass_scratch(RenderArgs &a, int views, bool single) {
     const bool fixed = capturing();
     const size_t nv = static_cast<size_t>(views), px = fixed ? nv * height * width : pixels();
     if (px > static_cast<size_t>(INT32_MAX)) return false;
+    if (!single && passes.refused != 0 && px >= passes.refused) return false;
     auto have = [&](auto &buf, size_t count) {
         if (fixed) return buf.n >= count;
         buf.ensure(count);
@@ -1021,7 +1027,13 @@ bool Renderer::pass_scratch(RenderArgs &a, int views, bool single) {
         if (!single) ok = ok && have(passes.rng, px) && have(passes.sum, px) && have(passes.visible, px);
         if (!ok) return false;
     } catch (const CudaFailure &) {
+        // Nothing per pixel stays behind for a kernel that does not use it, and so many pixels are not tried again until
+        // ngb_set_rows. (No capture holds these arrays: had they been there for the whole image, none had to grow.)
         cudaGetLastError();
+        if (!single) {
+            passes.release_pixels();
+            passes.refused = px;
+        }
         return false;
     }
     if (!a.basis_given) a.camera_basis = passes.basis.p;
@@ -1104,11 +1116,7 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
     const bool single = (outputs & NGB_OUTPUT_RGB) == 0 || one_pass(a, params.light_count);
     bool tiles = uneven ? persistent_ok
         : (kernel_choice == 3 || kernel_choice == 0 || (view && kernel_choice == 2 && persistent_ok));
-    // The per-pixel kernel needs no scratch: pictures that the tile kernels take several passes for go to it where the
-    // passes' scratch cannot be had.
-    if (tiles && !persistent_ok) tiles = pass_scratch(a, views, single);
-    const bool in_passes = tiles && !persistent_ok;
-    const bool persistent = !view && !tiles && persistent_ok && (kernel_choice == 0 || kernel_choice == 2);
+    // What any kernel needs comes before the passes' scratch.
     if (view && a.rgb) {
         a.radiance = view_radiance.ensure(pixels());
         if (view_accum.n < pixels()) {
@@ -1117,6 +1125,11 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         }
         view_argb.ensure(pixels());
     }
+    // The per-pixel kernel needs no scratch: pictures that the tile kernels take several passes for go to it where the
+    // passes' scratch cannot be had.
+    if (tiles && !persistent_ok) tiles = pass_scratch(a, views, single);
+    const bool in_passes = tiles && !persistent_ok;
+    const bool persistent = !view && !tiles && persistent_ok && (kernel_choice == 0 || kernel_choice == 2);
     require(!uneven || tiles, "worlds of uneven sizes render with one sample per pixel, at most one light and no "
         "reflective material");
     // Inside a CUDA graph capture the timing events would be graph nodes whose times cannot be read: the
@@ -1724,6 +1737,7 @@ int ngb_set_rows(ngb_renderer *h, int32_t first, int32_t count) {
             ") are not a non-empty range of the image's " + std::to_string(r.height) + " rows");
         r.band_first = first;
         r.band_rows = count == r.height ? 0 : count;
+        r.passes.refused = 0;
     });
 }
 

@@ -117,3 +117,30 @@ def test_failed_mesh_rebuild_can_be_made_again(torch_cuda):
     _, failures = until_it_works(lambda: r.update_mesh(0, v))
     assert failures >= 1
     assert same(r.render(wl.cameras, wl.fov, 1, **ALL), want)
+
+
+@pytest.mark.parametrize("k", range(12))
+def test_a_picture_whose_scratch_fails_is_drawn_without_it(torch_cuda, k):
+    """Two samples, two lights and mirrors take passes with scratch: four small arrays, then eight of a value per pixel.
+    Where the k-th fails the per-pixel kernel draws the picture, nothing per pixel stays allocated, and the passes are not
+    tried again until the rows are set."""
+    from test_gpu_sample_passes import images, scene
+    w, h, worlds, instances = 40, 32, 3, 6
+    r, cams = scene(worlds, instances, 2, True, w, h)
+    want = images(r, cams, 1, 2, rgb=True)["rgb"]             # the per-pixel kernel, and the arrays every render needs
+    pixels = want[..., 0].size
+    small = 48 * worlds + 8 * worlds * instances + 8 * 32     # per view, and the queue counters (an upper bound)
+    before = ng.device_bytes()
+    ng.inject_allocation_failure(k)
+    try:
+        got = images(r, cams, 0, 2, rgb=True)["rgb"]
+    finally:
+        ng.inject_allocation_failure(-1)
+    assert np.array_equal(got, want)
+    assert ng.device_bytes() - before <= small
+    assert np.array_equal(images(r, cams, 0, 2, rgb=True)["rgb"], want)
+    assert ng.device_bytes() - before <= small
+    r.set_rows(0, h)
+    passes = images(r, cams, 0, 2, rgb=True)["rgb"]
+    assert ng.device_bytes() - before >= 70 * pixels
+    assert (passes != want).any(-1).sum() <= pixels * 1e-4
