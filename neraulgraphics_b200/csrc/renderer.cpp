@@ -639,12 +639,17 @@ void Renderer::wait_times() {
     if (!timing_pending) return;
     if (times_id == 0) return wait(ev_stop, timeout);
     const auto start = std::chrono::steady_clock::now();
-    for (;;) {
-        // Read aside of the stream the render was queued on, until its last warp has left its number.
+    for (bool ended = false;;) {
+        // Read aside of the stream the render was queued on, until its last warp has left its number, and once more: the
+        // number is the last to be written, but a copy that met it may have read the times before it earlier.
         CK(cudaMemcpyAsync(host_times, times.p, sizeof(RenderTimes), cudaMemcpyDeviceToHost, own_stream));
         CK(cudaEventRecord(ev_done, own_stream));
         wait(ev_done, timeout);
-        if (host_times->id == times_id) return;
+        if (host_times->id == times_id) {
+            if (ended) return;
+            ended = true;
+            continue;
+        }
         if (std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count() > timeout)
             throw Timeout("the GPU work did not finish within " + std::to_string(timeout) + " seconds");
         std::this_thread::sleep_for(std::chrono::microseconds(20));

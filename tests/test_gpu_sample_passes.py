@@ -111,3 +111,17 @@ def test_stage_times_of_one_pass(lights, rgb):
         stages = r.last_stage_ms
         assert len(stages) == 3 and stages[0] > 0.0 and (stages[1] > 0.0) == rgb and (stages[2] > 0.0) == (rgb and lights == 1)
         assert abs(sum(stages) - r.last_kernel_ms) <= 1e-5 and r.last_kernel_ms < 50.0
+
+
+def test_times_read_while_the_render_runs_are_whole():
+    import torch
+    r, cams = scene(64, 8, 1, False, 64, 64)
+    dev = torch.from_numpy(cams).cuda()
+    into = {"rgb": torch.zeros((64, 64, 64, 3), dtype=torch.uint8, device="cuda")}
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(200):
+        with torch.cuda.stream(stream):
+            r.render(dev, 1.0, 1, rgb=True, into=into)
+        stages, ms = r.last_stage_ms, r.last_kernel_ms  # a poll that may meet the last warp's writes
+        assert len(stages) == 3 and min(stages) > 0.0 and abs(sum(stages) - ms) <= 1e-5 and ms < 50.0
