@@ -1181,14 +1181,11 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         if (in_passes) CK(cudaStreamWaitEvent(stream, passes.done, timed ? 0 : cudaEventWaitExternal));
         CK(launch_render_tiles(params, a, in_passes ? passes.counters.p : work_counter.p, shape, stream));
         if (in_passes) CK(cudaEventRecordWithFlags(passes.done, stream, timed ? 0 : cudaEventRecordExternal));
-        stages = by_kernels ? 3 : 1;
     } else if (persistent) {
         a.camera_basis = camera_basis.ensure(3 * static_cast<size_t>(views));
         CK(launch_render_persistent(params, a, reinterpret_cast<int *>(work_counter.p), tuning, stream));
-        stages = 1;
     } else {
         CK(launch_render(params, a, stream));
-        stages = 1;
     }
     if (a.radiance)
         CK(launch_accumulate(a.radiance, view_accum.p, frame, static_cast<long long>(pixels()), srgb_table.p,
@@ -1198,6 +1195,7 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
         CK(launch_mark_end(a, stream));
     }
     if (timed) {
+        stages = by_kernels ? 3 : 1;
         times_id = by_kernels ? a.time_id : 0;
         if (!by_kernels) CK(cudaEventRecord(ev_stop, stream));
         timing_pending = true;

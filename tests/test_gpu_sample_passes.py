@@ -125,3 +125,23 @@ def test_times_read_while_the_render_runs_are_whole():
             r.render(dev, 1.0, 1, rgb=True, into=into)
         stages, ms = r.last_stage_ms, r.last_kernel_ms  # a poll that may meet the last warp's writes
         assert len(stages) == 3 and min(stages) > 0.0 and abs(sum(stages) - ms) <= 1e-5 and ms < 50.0
+
+
+@pytest.mark.parametrize("spp", [1, 2])
+def test_a_capture_keeps_the_times_of_the_render_before_it(spp):
+    import torch
+    r, cams = scene(4, 8, 1, False, 64, 64)
+    dev = torch.from_numpy(cams).cuda()
+    into = {"rgb": torch.zeros((4, 64, 64, 3), dtype=torch.uint8, device="cuda")}
+    r.render(dev, 1.0, spp, rgb=True, into=into)
+    torch.cuda.synchronize()
+    r.render(dev, 1.0, 1, rgb=True, into=into)
+    want = r.last_stage_ms, r.last_kernel_ms
+    assert len(want[0]) == 3
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        r.render(dev, 1.0, spp, rgb=True, into=into)
+    g.replay()
+    torch.cuda.synchronize()
+    assert (r.last_stage_ms, r.last_kernel_ms) == want
+    del g
