@@ -1239,7 +1239,7 @@ void Renderer::cast_rays(const float *o, const float *d, int rays_per_world, flo
     if (timed) CK(cudaEventRecord(ev_start, stream));
     // Automatic: warp packets (a 64 x 2048 LiDAR sweep of 100,000 instances 0.37 against 0.58 ms for the persistent
     // kernel's lane-refilling walk; 1024 worlds of 20 instances: 720-beam scans 0.13 against 0.27 ms, 64-beam 0.074
-    // against 0.138, rays in all directions 0.35 against 0.37); the per-thread kernel when the per-pixel kernel is
+    // against 0.138, rays in all directions 0.245 against 0.36); the per-thread kernel when the per-pixel kernel is
     // chosen, the persistent one when it is; or as ngb_set_ray_kernel says.
     const int mode = ray_kernel != 0 ? ray_kernel : kernel_choice == 1 ? 1 : kernel_choice == 2 ? 2 : 3;
     if (mode == 1) CK(launch_rays(params, a, stream));

@@ -50,3 +50,27 @@ def test_default_walks_give_the_per_thread_kernels_hits(worlds, instances, rays,
     for name in want:
         differ = (got[name] != want[name]).reshape(worlds * rays, -1).any(-1).sum()
         assert differ <= worlds * rays * 1e-4, (name, differ)
+
+
+@pytest.mark.parametrize("rays,dead", [(7, ()), (16, ()), (48, ()), (32, (16,)), (31, (16, 20)), (2, ())])
+def test_the_walk_does_not_depend_on_where_a_sensor_faces(rays, dead):
+    """Two meshes share a square; rays from the left enter the first's box before the second's, rays from the right the
+    other way round. Which of the two coincident surfaces a ray reports shows which walk its warp took, so a scene
+    turned round, sensor and all, has to report the same ones."""
+    square = np.array([(-1, -1, -1), (1, -1, -1), (1, 1, -1), (-1, 1, -1)], np.float32)
+    fins = [np.array([(s * 3, 0.9, 0), (s * 3, 0.8, 0), (s * 3, 0.9, -0.1)], np.float32) for s in (-1, 1)]
+    index = np.array([0, 1, 2, 0, 2, 3, 4, 5, 6], np.uint32)
+    side = np.where(np.arange(rays) % 3 == 2, 1.0, -1.0)  # two rays in three from the left
+    o = np.stack([2.2 * side, np.linspace(-0.4, 0.4, rays), np.ones(rays)], -1)[None].astype(np.float32)
+    d = np.stack([-0.6 * side, np.zeros(rays), np.full(rays, -0.8)], -1)[None].astype(np.float32)
+    d[:, list(dead)] = 0.0
+    found = []
+    for turn in (1.0, -1.0):  # half a turn about y
+        t = np.array([turn, 1.0, turn], np.float32)
+        r = ng.BatchRenderer(8, 8, 1, 1, meshes=[ng.Mesh(np.concatenate([square, f]) * t, index) for f in fins],
+                             instances=[ng.Instance(0), ng.Instance(1)])
+        found.append(r.cast_rays(o * t, d * t, 10.0))
+    live = ~np.isin(np.arange(rays), dead)
+    assert np.isfinite(found[0]["distance"][0]).tolist() == live.tolist()
+    assert np.array_equal(found[0]["distance"], found[1]["distance"])
+    assert np.array_equal(found[0]["object_id"], found[1]["object_id"])
