@@ -317,7 +317,8 @@ int ngb_set_sync(ngb_renderer *r, int32_t synchronous, double timeout_seconds);
  * passes' scratch (77 bytes per pixel, kept) cannot be had: no memory (not tried again for as many pixels until
  * ngb_set_rows), or a stream capture before any such render of the whole image. 1: the per-pixel kernel.
  * 2: the persistent kernel where it applies (what takes one pass), else the per-pixel kernel.
- * Ray queries (ngb_cast_rays), unless ngb_set_ray_kernel chose otherwise, take warp packets (kernel 0 or 3), the
+ * Ray queries (ngb_cast_rays), unless ngb_set_ray_kernel chose otherwise, take warp packets (kernel 0 or 3; in more than
+ * 32768 worlds of at most 256 instances with up to one ray, and at most 16, per 8192 worlds the persistent kernel), the
  * persistent kernel in its shape (kernel 2), or the per-thread ray kernel (kernel 1).
  * With kernel 3 the call sets the tile kernel's shape: threads_per_block and registers as one of 128/48,
  * 128/56, 128/64, 128/80, 256/64 (default 128/56, 128/64 for worlds above 256 instances); refill_lanes and

@@ -74,3 +74,41 @@ def test_the_walk_does_not_depend_on_where_a_sensor_faces(rays, dead):
     assert np.isfinite(found[0]["distance"][0]).tolist() == live.tolist()
     assert np.array_equal(found[0]["distance"], found[1]["distance"])
     assert np.array_equal(found[0]["object_id"], found[1]["object_id"])
+
+
+def crowd(worlds, rays):
+    import torch
+    rng = np.random.default_rng(worlds + rays)
+    r = ng.BatchRenderer(8, 8, worlds, 1, meshes=[ng.make_icosphere(0.5, 1)], instances=[ng.Instance(0)] * 2)
+    m = np.zeros((worlds, 2, 3, 4), np.float32)
+    m[..., [0, 1, 2], [0, 1, 2]] = 1.0
+    m[..., 3] = rng.uniform(-1.5, 1.5, size=(worlds, 2, 3))
+    r.set_instance_transforms(m)
+    d = rng.normal(size=(worlds, rays, 3)).astype(np.float32)
+    return r, torch.from_numpy(np.zeros_like(d)).cuda(), torch.from_numpy(d).cuda()
+
+
+@pytest.mark.parametrize("worlds,rays", [(32768, 4), (32769, 4), (32769, 5), (40961, 5), (65536, 9)])
+def test_many_worlds_of_few_rays_give_the_per_thread_kernels_hits(worlds, rays):
+    import torch
+    r, o, d = crowd(worlds, rays)
+    got = r.cast_rays(o, d, 5.0)
+    r.set_ray_kernel(1)
+    want = r.cast_rays(o, d, 5.0)
+    torch.cuda.synchronize()
+    assert int(torch.isfinite(want["distance"]).sum()) > worlds * rays // 20
+    for name in want:
+        differ = (got[name] != want[name]).reshape(worlds * rays, -1).any(-1).sum().item()
+        assert differ <= worlds * rays * 1e-4, (name, differ)
+
+
+def test_many_worlds_of_one_ray_take_no_longer_than_on_the_persistent_kernel():
+    r, o, d = crowd(262144, 1)
+    ms = {}
+    for kernel in (0, 2, 0, 2):
+        r.set_ray_kernel(kernel)
+        for _ in range(5):
+            r.cast_rays(o, d, 5.0)
+            r.synchronize()
+            ms[kernel] = min(r.last_kernel_ms, ms.get(kernel, 1e9))
+    assert ms[0] <= 1.5 * ms[2], ms  # packets of one ray each: 3.8 times
