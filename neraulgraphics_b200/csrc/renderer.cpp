@@ -293,6 +293,17 @@ struct Renderer {
     void cast_rays(const float *o, const float *d, int rays_per_world, float max_distance, int memory, ngb_ray_hits *out,
         float *distance, float *normal, int32_t *ids);
     bool pass_scratch(RenderArgs &a, int views, bool single);
+    // Whether the images are so small and coarse that passes lose to the per-pixel kernel, whose one launch then has room
+    // for every ray at once: a pass is as long as its longest walk, and a warp's pixels lie so far apart that they share
+    // little of theirs. Per-pixel time over the passes', two samples and one light or one and two, by instances a world:
+    // 5 at 8 x 8 pixels 0.7 to 1.3, at 16 x 16 0.9 to 1.8; 250 at 8 x 8 0.7 to 0.9, at 16 x 16 0.95 to 1.4; 300 at
+    // 17 x 17 0.8 to 1.1, at 32 x 32 1.0 to 1.3; 1000 at 24 x 24 0.8 to 0.95, at 48 x 48 0.95 to 1.2; 20,000 at 64 x 64
+    // 0.8, at 160 x 160 0.95 to 1.1; 100,000 at 128 x 128 0.8, at 256 x 256 1.1. Many views fill the GPU either way: 512
+    // of 8 x 8 pixels and 20 instances 1.2 to 1.6, 64 of 24 x 24 and 300 1.1 to 1.2.
+    bool coarse() const {
+        const long long limit = per_world <= TILE_MAX_INSTANCES ? 64 + 3LL * per_world / 4 : 512 + 3LL * per_world / 5;
+        return pixels() < 32768 && static_cast<long long>(width) * height < limit;
+    }
     int rows() const { return band_rows > 0 ? band_rows : height; }
     size_t pixels() const {
         return uneven ? static_cast<size_t>(total_pixels) : static_cast<size_t>(worlds) * cpw * rows() * width;
@@ -1132,7 +1143,7 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
     }
     // The per-pixel kernel needs no scratch: pictures that the tile kernels take several passes for go to it where the
     // passes' scratch cannot be had.
-    if (tiles && !persistent_ok) tiles = pass_scratch(a, views, single);
+    if (tiles && !persistent_ok) tiles = !(kernel_choice == 0 && coarse()) && pass_scratch(a, views, single);
     const bool in_passes = tiles && !persistent_ok;
     const bool persistent = !view && !tiles && persistent_ok && (kernel_choice == 0 || kernel_choice == 2);
     require(!uneven || tiles, "worlds of uneven sizes render with one sample per pixel, at most one light and no "

@@ -145,3 +145,25 @@ def test_a_capture_keeps_the_times_of_the_render_before_it(spp):
     torch.cuda.synchronize()
     assert (r.last_stage_ms, r.last_kernel_ms) == want
     del g
+
+
+@pytest.mark.parametrize("instances,worlds,size,coarse", [(8, 1, 8, True), (8, 1, 9, False), (256, 4, 15, True),
+                                                          (256, 4, 16, False), (257, 2, 25, True), (257, 2, 26, False),
+                                                          (300, 56, 24, True), (300, 57, 24, False)])
+def test_coarse_pictures_take_the_per_pixel_kernel(instances, worlds, size, coarse):
+    r, cams = scene(worlds, instances, 2, True, size, size)
+    want = images(r, cams, 1, 2, rgb=True, depth=True)
+    before = ng.device_bytes()
+    got = images(r, cams, 0, 2, rgb=True, depth=True)
+    pixels = worlds * size * size
+    if coarse:  # it needs no scratch
+        assert ng.device_bytes() == before
+        assert all(np.array_equal(got[k], want[k]) for k in want)
+    else:
+        assert ng.device_bytes() - before >= 70 * pixels
+    forced = images(r, cams, 3, 2, rgb=True, depth=True)
+    for other in (got, forced):
+        for k in want:
+            differ = (other[k] != want[k]).reshape(pixels, -1).any(-1).sum()
+            assert differ <= max(pixels * 1e-4, 1), (k, differ)
+    assert ng.device_bytes() - before >= 70 * pixels
