@@ -14,7 +14,7 @@
 //   d(A^-T) = -A^-T dA^T A^-T, dp = A^-1 (dP - dA p - db), (du, dv) = (a1 . dp, a2 . dp) with a1, a2 the dual
 //   basis of (e1, e2) in the triangle's plane.
 // The kernel applies their transposes to the upstream gradients of D and N, pixel by pixel, and sums them
-// per instance and per camera: first in shared memory (one CTA is one 16 x 8 tile of one view, so all its
+// per instance and per camera: first in shared memory (one CTA is one tile of one view, so all its
 // pixels share a camera and a world), then into the caller's arrays with one atomic per entry and CTA.
 #include "device.cuh"
 #include "kernels.h"
@@ -22,11 +22,15 @@
 namespace ngb {
 namespace {
 
-// What bounds the kernel is its arithmetic and the waits at the CTA's barriers, not memory (0.6 GB, 0.09 ms): tiles of 128
-// pixels against 256, 1024 views of
-// 128 x 128: 0.59 -> 0.56 ms.
-constexpr int ADJ_W = 16, ADJ_H = 8;
-constexpr int ADJ_THREADS = ADJ_W * ADJ_H;
+// A CTA's tile: 16 x ROWS pixels. What bounds the kernel is the latency of its loads and the waits at the CTA's barriers,
+// not memory (0.6 GB, 0.09 ms at 1024 views of 128 x 128): small CTAs wait less, but each clears and flushes its world's
+// sums, whose shared memory also limits how many are resident. Backward of 128 x 128 views, 256 against 128 pixels a
+// CTA: 1024 worlds of 12 instances 685 against 654 us, 512 of 100 544 against 531, 256 of 256 354 against 344, of 400
+// 366 against 372, 128 of 512 226 against 241, of 1000 245 against 371, 64 of 1500 (whose sums are in global memory) 137
+// against 132.
+constexpr int ADJ_W = 16;
+constexpr int ADJ_SHARED_WORLD = 1024;  // the largest world whose sums are in shared memory (48 KB)
+inline bool large_tiles(int per_world) { return per_world > 256 && per_world <= ADJ_SHARED_WORLD; }
 
 struct M3 {
     float a[3][3];
@@ -105,13 +109,15 @@ __device__ __forceinline__ float warp_sums12(const float *in, int lane) {
     return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-__global__ void __launch_bounds__(ADJ_THREADS, 8) depth_normal_adjoint_kernel(const __grid_constant__ SceneParams s,
+template <int ROWS>
+__global__ void __launch_bounds__(ADJ_W * ROWS, 64 / ROWS) depth_normal_adjoint_kernel(const __grid_constant__ SceneParams s,
     const AdjointArgs a, int tiles_x, int tiles_per_view, bool shared_sums) {
+    constexpr int ADJ_THREADS = ADJ_W * ROWS;
     extern __shared__ float sums[];  // per instance of the world 12, then the camera's 12
     const int view = blockIdx.x / tiles_per_view;
     const int q = blockIdx.x % tiles_per_view;
     const int x = (q % tiles_x) * ADJ_W + threadIdx.x % ADJ_W;
-    const int y = a.row_first + (q / tiles_x) * ADJ_H + threadIdx.x / ADJ_W;
+    const int y = a.row_first + (q / tiles_x) * ROWS + threadIdx.x / ADJ_W;
     const int world = view / a.cameras_per_world;
     const int P = s.per_world;
     float *cam_sum = sums + (shared_sums ? 12 * P : 0);
@@ -269,22 +275,26 @@ __global__ void __launch_bounds__(ADJ_THREADS, 8) depth_normal_adjoint_kernel(co
         atomicAdd(a.grad_cameras + 12LL * view + threadIdx.x, cam_sum[threadIdx.x]);
 }
 
-}  // namespace
-
-cudaError_t launch_depth_normal_adjoint(const SceneParams &s, const AdjointArgs &a, cudaStream_t stream) {
-    const int tiles_x = (a.width + ADJ_W - 1) / ADJ_W, tiles_y = (a.rows + ADJ_H - 1) / ADJ_H;
+template <int ROWS>
+cudaError_t launch_rows(const SceneParams &s, const AdjointArgs &a, cudaStream_t stream) {
+    const int tiles_x = (a.width + ADJ_W - 1) / ADJ_W, tiles_y = (a.rows + ROWS - 1) / ROWS;
     const long long blocks = static_cast<long long>(tiles_x) * tiles_y * a.views;
     if (blocks == 0) return cudaSuccess;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    // Per-instance sums in shared memory for worlds of up to 1024 instances (48 KB), else straight to global.
-    const bool shared_sums = s.per_world <= 1024;
+    const bool shared_sums = s.per_world <= ADJ_SHARED_WORLD;
     const size_t smem = sizeof(float) * ((shared_sums ? 12 * static_cast<size_t>(s.per_world) : 0) + 12);
-    cudaError_t e = cudaFuncSetAttribute(depth_normal_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(depth_normal_adjoint_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
         static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    depth_normal_adjoint_kernel<<<static_cast<unsigned>(blocks), ADJ_THREADS, smem, stream>>>(s, a, tiles_x,
+    depth_normal_adjoint_kernel<ROWS><<<static_cast<unsigned>(blocks), ADJ_W * ROWS, smem, stream>>>(s, a, tiles_x,
         tiles_x * tiles_y, shared_sums);
     return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_depth_normal_adjoint(const SceneParams &s, const AdjointArgs &a, cudaStream_t stream) {
+    return large_tiles(s.per_world) ? launch_rows<16>(s, a, stream) : launch_rows<8>(s, a, stream);
 }
 
 }  // namespace ngb

@@ -22,18 +22,21 @@ from adjoint_ref import reference_depth_normals, rel_err, silhouette_free
 pytestmark = pytest.mark.gpu
 
 
-def make(worlds=4, width=48, height=40, seed=3):
-    wl = workloads.differentiable_worlds(worlds=worlds, width=width, height=height, seed=seed)
+def make(worlds=4, width=48, height=40, seed=3, per_world=12):
+    wl = workloads.differentiable_worlds(worlds=worlds, per_world=per_world, width=width, height=height, seed=seed)
     d = wl.desc
     r = ng.BatchRenderer(d.width, d.height, d.world_count, 1, d.spheres, d.lights, d.floor, d.meshes, d.instances,
                          device="cuda:0")
     return wl, r
 
 
-def test_adjoint_is_the_float64_reference(torch_cuda):
+# And ragged images at the instance counts where the kernel's tiles grow (257) and its sums leave shared memory (1025).
+@pytest.mark.parametrize("args", [{}, *({"worlds": 2, "width": 33, "height": 21, "per_world": p} for p in (256, 257, 1024, 1025))],
+                         ids=lambda a: str(a.get("per_world", 12)))
+def test_adjoint_is_the_float64_reference(torch_cuda, args):
     torch = torch_cuda
     from neraulgraphics_b200.autodiff import render_depth_normals
-    wl, r = make()
+    wl, r = make(**args)
     mats = torch.from_numpy(wl.matrices).cuda().requires_grad_()
     cams = torch.from_numpy(wl.cameras).cuda().requires_grad_()
     depth, normals = render_depth_normals(r, mats, cams, wl.fov)
