@@ -10,8 +10,9 @@
 // memory: compose the matrix, invert it, box it, reduce the world's centre bounds, make the keys, rank-sort
 // them, emit the Karras nodes, and refit the boxes bottom-up with shared-memory atomics. The only nodes a
 // group cannot finish are the inter-world ones (never traversed: every ray starts at its world's root);
-// their links are emitted by the group that owns their index, and a second small launch fits their boxes
-// by climbing from the world roots, as fit_boxes does (cuda_tlas.cuh:179-196).
+// their links are emitted by the group that owns their index, and their boxes are made by the build's last CTA (up to
+// 128 worlds), by a launch of one CTA that joins blocks of worlds (up to 2048), or by a launch that climbs from
+// the world roots, as fit_boxes does (cuda_tlas.cuh:179-196).
 #include <climits>
 
 #include "device.cuh"
@@ -221,9 +222,14 @@ __device__ __forceinline__ void fit_world(int w, const int *roots, const int *pa
     }
 }
 
-// The inter-world nodes' boxes by one CTA, for at most a world per thread: the worlds' root boxes in shared memory, and each
-// node's box from those of the worlds that its range covers. (A climb's level takes about 1.2 us of fences, atomics and
-// dependent loads, and 16 worlds take four; here no thread waits for another's node.)
+// The inter-world nodes' boxes by one CTA, for at most FIT_INSIDE worlds (a world per thread): the worlds' root boxes in
+// shared memory, and each node's box from those of the worlds that its range covers. (A climb's level takes about 1.2 us
+// of fences, atomics and dependent loads, and 16 worlds take four; here no thread waits for another's node.) One thread
+// joins every world's box for the root, so a launch of fit_blocks_kernel is faster for many worlds, whatever the CTA
+// holds. Builds of 300 and 700 instances a world, joined here against there: 96 worlds 38 against 41 and 59 against 62
+// us, 128 38 against 41 and 59 against 62, 192 48 against 52 and 98 against 96, 256 50 against 49 and 100 against 97,
+// 512 81 against 69 and 183 against 170.
+constexpr int FIT_INSIDE = 128;
 __device__ __forceinline__ void fit_worlds_inside(const BuildArgs &a, float *boxes, int threads) {
     const int w = threadIdx.x, n = static_cast<int>(a.n);
     if (w < a.worlds) {
@@ -460,9 +466,9 @@ __global__ void __launch_bounds__(G < 128 ? 128 : G) build_worlds_kernel(const B
         }
     }
 
-    // The last CTA to come here has every other's nodes before it. (At most a world per thread: the build
-    // and the fit of 16 worlds 23 -> 12 us, one launch for two.)
-    if (a.built == nullptr || a.worlds < 2 || a.worlds > CTA) return;
+    // The last CTA to come here has every other's nodes before it. (The build and the fit of 16 worlds 23 -> 12 us, one
+    // launch for two.)
+    if (a.built == nullptr || a.worlds < 2 || a.worlds > FIT_INSIDE) return;
     __shared__ int last;
     __threadfence();
     __syncthreads();
@@ -481,6 +487,8 @@ __global__ void __launch_bounds__(G < 128 ? 128 : G) build_worlds_kernel(const B
 // all its worlds with instances lie between them). Twelve short steps where the climbs took as many rounds of fences,
 // atomics and dependent loads: 25 -> 15 us for 1024 worlds; for 4096 it is the
 // climbs, spread over the chip, that are faster, 30 against 40 us.
+// (Between those two counts the line is not measured; nothing jumps there: 2000 to 4096 worlds of 20 instances build in 54
+// to 58 us.)
 constexpr int FIT_THREADS = 1024, FIT_WORLDS = 2048;
 __global__ void __launch_bounds__(FIT_THREADS, 1) fit_blocks_kernel(const BuildArgs a) {
     extern __shared__ float fit_smem[];
@@ -946,8 +954,7 @@ cudaError_t launch_build_worlds(const BuildArgs &a, cudaStream_t stream) {
     default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
-    const int threads = build_group_size(a.per_world) < 128 ? 128 : build_group_size(a.per_world);
-    if (a.worlds > 1 && a.built != nullptr && a.worlds <= threads) return cudaSuccess;  // the build fitted them itself
+    if (a.worlds > 1 && a.built != nullptr && a.worlds <= FIT_INSIDE) return cudaSuccess;  // the build fitted them itself
     if (a.worlds > 1 && a.worlds <= FIT_WORLDS) {
         const size_t smem = sizeof(float) * 6 * (a.worlds + (a.worlds + 1) / 2);
         e = cudaFuncSetAttribute(fit_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

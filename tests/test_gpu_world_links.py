@@ -21,7 +21,7 @@ def placed(rng, shape):
 
 @pytest.mark.parametrize("worlds,instances", [(1, 2), (2, 1), (3, 1), (7, 1), (64, 1), (127, 1), (128, 1), (129, 1), (1024, 1), (2047, 2), (2049, 1), (5, 2), (6, 3),
                                               (33, 5), (128, 3), (129, 3), (9, 31), (4, 32), (5, 33), (3, 64), (17, 100), (1500, 2),
-                                              (3, 200), (2, 513)])
+                                              (3, 200), (2, 513), (128, 300), (129, 300), (129, 200)])
 def test_batched_trees_are_the_oracles(worlds, instances):
     rng = np.random.default_rng(worlds * 1000 + instances)
     m = placed(rng, (worlds, instances))
