@@ -210,8 +210,9 @@ float surface(const Box &b) {
 }
 
 int bin_index(float c, float lo, float scale) {
-    const int b = static_cast<int>((c - lo) * scale);
-    return b < BINS - 1 ? b : BINS - 1;
+    // Compared before the conversion: an extent below 16 / FLT_MAX has an infinite scale, and no int holds that or 0 x inf.
+    const float f = (c - lo) * scale;
+    return f >= static_cast<float>(BINS - 1) ? BINS - 1 : f > 0.0f ? static_cast<int>(f) : 0;
 }
 
 // A node while the tree is built: its triangle range in `order`, its depth, its box and its first child in

@@ -378,3 +378,28 @@ def test_geom_matrices_are_the_compose_kernels_products():
                 for c in range(3):
                     assert got[w, i, row, c] == np.float32(xmat[w, g, row, c] * scale[i, c])
                 assert got[w, i, row, 3] == xpos[w, g, row]
+
+
+def test_meshes_of_the_smallest_extents_have_trees():
+    """Centres closer than 16 / FLT_MAX: the bins' scale is infinite. Every triangle is in one leaf, every box holds its
+    triangles."""
+    import neraulgraphics_b200 as ng
+    rng = np.random.default_rng(1)
+    for triangles in (5, 64, 700):
+        fall = 0.5 ** np.linspace(100.0, 148.0, triangles)
+        v = ((rng.uniform(-1.0, 1.0, size=(triangles, 3, 3)) + 1.5) * fall[:, None, None]).astype(np.float32)
+        tree = ng.build_meshes([ng.Mesh(v.reshape(-1, 3), np.arange(3 * triangles))])
+        assert sorted(tree["triangle_index"]) == list(range(triangles))
+        nodes = tree["nodes"].reshape(-1, 8)
+        box = nodes.view(np.float32)
+        seen, below = 0, [0]
+        while below:
+            n = below.pop()
+            first, count = nodes[n, 3], nodes[n, 7]
+            if count == 0:
+                below += [first, first + 1]
+                continue
+            t = v[tree["triangle_index"][first:first + count]]
+            assert (t >= box[n, :3]).all() and (t <= box[n, 4:7]).all()
+            seen += count
+        assert seen == triangles
