@@ -299,10 +299,12 @@ struct Renderer {
     // 5 at 8 x 8 pixels 0.7 to 1.3, at 16 x 16 0.9 to 1.8; 250 at 8 x 8 0.7 to 0.9, at 16 x 16 0.95 to 1.4; 300 at
     // 17 x 17 0.8 to 1.1, at 32 x 32 1.0 to 1.3; 1000 at 24 x 24 0.8 to 0.95, at 48 x 48 0.95 to 1.2; 20,000 at 64 x 64
     // 0.8, at 160 x 160 0.95 to 1.1; 100,000 at 128 x 128 0.8, at 256 x 256 1.1. Many views fill the GPU either way: 512
-    // of 8 x 8 pixels and 20 instances 1.2 to 1.6, 64 of 24 x 24 and 300 1.1 to 1.2.
+    // of 8 x 8 pixels and 20 instances 1.2 to 1.6, 64 of 24 x 24 and 300 1.1 to 1.2. By the whole images, so that a band of
+    // rows is drawn by the kernel that draws them whole.
     bool coarse() const {
         const long long limit = per_world <= TILE_MAX_INSTANCES ? 64 + 3LL * per_world / 4 : 512 + 3LL * per_world / 5;
-        return pixels() < 32768 && static_cast<long long>(width) * height < limit;
+        const long long image = static_cast<long long>(width) * height;
+        return image < limit && image * worlds * cpw < 32768;
     }
     int rows() const { return band_rows > 0 ? band_rows : height; }
     size_t pixels() const {

@@ -167,3 +167,11 @@ def test_coarse_pictures_take_the_per_pixel_kernel(instances, worlds, size, coar
             differ = (other[k] != want[k]).reshape(pixels, -1).any(-1).sum()
             assert differ <= max(pixels * 1e-4, 1), (k, differ)
     assert ng.device_bytes() - before >= 70 * pixels
+    # A band of rows takes the whole image's kernel.
+    r, cams = scene(worlds, instances, 2, True, size, size)
+    r.set_rows(4, 4)
+    images(r, cams, 1, 2, rgb=True, depth=True)
+    before = ng.device_bytes()
+    band = images(r, cams, 0, 2, rgb=True, depth=True)
+    assert (ng.device_bytes() == before) == coarse
+    assert all(np.array_equal(band[k], got[k][:, 4:8]) for k in band)
