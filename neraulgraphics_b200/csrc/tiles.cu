@@ -41,7 +41,7 @@ constexpr int WALK_STACK = 64;      // a mesh's tree is at most 60 deep
 
 // A tile's candidate instances as its warp holds them: each one's position in its world's run of sorted
 // leaves and the distance below which no camera ray of the tile can enter its box, in the view's order of those
-// distances (view_order_kernel). CAP: the most instances a world holds (32 or TILE_MAX_INSTANCES).
+// distances (setup_kernel). CAP: the most instances a world holds (32 or TILE_MAX_INSTANCES).
 template <int CAP>
 struct WarpSmem {
     int leaf[CAP];           // the candidates' leaves, smallest entry bound first (the view's order)
@@ -1198,7 +1198,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) ray_packets_kernel(const 
         // ms), and so do up to half a warp's, which share too little (fans of 57 degrees in 16 to 4096 worlds of 1 to 200
         // instances: 12 to 16 rays 2 to 3 % faster alone).
         const unsigned rays = __ballot_sync(FULL, live);
-        const int middle_lane = __ffs(__ballot_sync(FULL, live && __popc(rays & ((1u << lane) - 1u)) == __popc(rays) / 2)) - 1;
+        const int half = (32 - __clz(rays)) >> 1, middle_lane = half + __ffs(rays >> half) - 1;
         const float3 middle = mk3(__shfl_sync(FULL, d.x, middle_lane), __shfl_sync(FULL, d.y, middle_lane),
             __shfl_sync(FULL, d.z, middle_lane));
         const bool together = __popc(rays) > 16 && __all_sync(FULL, !live || dot(d, middle) > 0.0f);
