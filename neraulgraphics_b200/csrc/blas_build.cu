@@ -51,6 +51,9 @@ __device__ __forceinline__ float area(const Box &b) {
     return 2.0f * (dx * dy + dy * dz + dz * dx);
 }
 
+// Bins per length, finite also for extents below 16 / FLT_MAX (as the host build's).
+__device__ __forceinline__ float bin_scale(float extent) { return fminf(static_cast<float>(BINS) / extent, 3.402823466e38f); }
+
 __device__ __forceinline__ int bin_of(float c, float lo, float scale) {
     const int b = static_cast<int>((c - lo) * scale);
     return b < 0 ? 0 : b < BINS - 1 ? b : BINS - 1;  // (never below 0 for finite vertices)
@@ -260,7 +263,7 @@ __device__ void split_node(const MeshBuildArgs &a, const MeshBuildScratch &t, in
     float best_cost = __int_as_float(0x7f800000);
     if (count > 1) {
         float scale[3];
-        for (int axis = 0; axis < 3; ++axis) scale[axis] = static_cast<float>(BINS) / (cb[3 + axis] - cb[axis]);
+        for (int axis = 0; axis < 3; ++axis) scale[axis] = bin_scale(cb[3 + axis] - cb[axis]);
         for (int i = begin + tid; i < end; i += THREADS) {
             const size_t p = t.order[i];
             int b[6];
@@ -302,7 +305,7 @@ __device__ void split_node(const MeshBuildArgs &a, const MeshBuildScratch &t, in
     int mid = begin + count / 2;
     if (best_axis >= 0) {
         const float lo = cb[best_axis];
-        const float scale = static_cast<float>(BINS) / (cb[3 + best_axis] - lo);
+        const float scale = bin_scale(cb[3 + best_axis] - lo);
         auto passes_item = [&](uint32_t p) {
             return bin_of(t.centre[3 * static_cast<size_t>(p) + best_axis], lo, scale) <= best_bin;
         };

@@ -209,10 +209,12 @@ float surface(const Box &b) {
     return 2.0f * (dx * dy + dy * dz + dz * dx);
 }
 
+// Bins per length. Finite also for extents below 16 / FLT_MAX: no int holds the bin of an infinite scale.
+float bin_scale(float extent) { return std::min(static_cast<float>(BINS) / extent, std::numeric_limits<float>::max()); }
+
 int bin_index(float c, float lo, float scale) {
-    // Compared before the conversion: an extent below 16 / FLT_MAX has an infinite scale, and no int holds that or 0 x inf.
-    const float f = (c - lo) * scale;
-    return f >= static_cast<float>(BINS - 1) ? BINS - 1 : f > 0.0f ? static_cast<int>(f) : 0;
+    const int b = static_cast<int>((c - lo) * scale);
+    return b < BINS - 1 ? b : BINS - 1;
 }
 
 // A node while the tree is built: its triangle range in `order`, its depth, its box and its first child in
@@ -242,7 +244,7 @@ Plane cheapest_plane(const Items &it, uint32_t begin, uint32_t end, const Box &c
     for (int axis = 0; axis < 3; ++axis) {
         const float extent = cbox.hi[axis] - cbox.lo[axis];
         if (!(extent > 0.0f)) continue;
-        const float scale = static_cast<float>(BINS) / extent;
+        const float scale = bin_scale(extent);
         Box bins[BINS];
         int count[BINS] = {};
         for (Box &b : bins) b = Box{{INF, INF, INF}, {-INF, -INF, -INF}};
@@ -299,7 +301,7 @@ void split(Items &it, std::vector<Draft> &drafts, size_t x) {
     uint32_t mid = begin + count / 2;
     if (plane.axis >= 0) {
         const float lo = cbox.lo[plane.axis];
-        const float scale = static_cast<float>(BINS) / (cbox.hi[plane.axis] - lo);
+        const float scale = bin_scale(cbox.hi[plane.axis] - lo);
         auto passes = [&](uint32_t i) {
             return bin_index(it.centre[3 * static_cast<size_t>(it.order[i]) + plane.axis], lo, scale) <= plane.bin;
         };
