@@ -386,11 +386,13 @@ int32_t ngb_world_count(const ngb_renderer *r);
 int32_t ngb_cameras_per_world(const ngb_renderer *r);
 int32_t ngb_view_count(const ngb_renderer *r);
 int32_t ngb_instances_per_world(const ngb_renderer *r);
-/* GPU time of the last render or ray query, from CUDA events around its launch (cuda_backend.cu:537-543). */
+/* GPU time of the last render or ray query that was not captured: of a render on the tile kernels in one pass from the
+ * GPU's global timer, read by its first and last kernels; of the others from CUDA events around their launches
+ * (cuda_backend.cu:537-543). */
 float ngb_last_kernel_ms(const ngb_renderer *r);
-/* The last render's GPU time by kernel, from CUDA events between its launches: *count = 3 for the tile
- * kernels (camera rays, shading, shadow rays), 1 for the others (the whole launch). Up to capacity entries are
- * written. No counterpart in the reference, which times the render as one launch. */
+/* The same time by kernel: *count = 3 for the tile kernels in one pass (camera rays, shading, shadow rays), 1 for the
+ * others, pictures in several passes among them (the whole render). Up to capacity entries are written. No counterpart
+ * in the reference, which times the render as one launch. */
 int ngb_last_stage_ms(ngb_renderer *r, float *ms, int32_t capacity, int32_t *count);
 
 /* ---- one view: the single-view Renderer ------------------------------------------------------------- */

@@ -113,7 +113,7 @@ struct RenderArgs {
     int basis_given;
     float4 *radiance;
     // The tile kernels' per-view candidate order (views x order_stride): instances by the eye's distance to their
-    // boxes, and those distances (see tiles.cu view_order_kernel).
+    // boxes, and those distances (see tiles.cu setup_kernel).
     int *view_order;
     float *view_bound;
     int order_stride;

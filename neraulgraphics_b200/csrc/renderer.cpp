@@ -1186,8 +1186,11 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
             if (!a.radiance && (!a.rgb || params.light_count == 1)) a.ended = ended;
             a.time_id = ++times_count;
         }
-        // Packet walks spill at 56 registers (100,000 instances at 1280 x 720: 1.206 ms, 1.158 at 64); candidate lists do
-        // not, and more warps serve them better (4096 worlds: 5.19 against 5.21).
+        // Packet walks spill (132 to 208 bytes stored a thread of the camera kernels at 56 registers, 44 to 120 at 64, 0 to
+        // 52 at 80) and are fastest at 64 whatever the render asks for. At 1280 x 720 with 56, 64 and 80: 2000 instances,
+        // colour 0.94, 0.92 and 0.95 ms, depth 0.417, 0.405 and 0.418, both and IDs 1.18, 1.16 and 1.19; 100,000: 1.23,
+        // 1.16 and 1.17, 0.580, 0.560 and 0.577, 1.48, 1.44 and 1.48. Candidate lists spill little (24 to 52 bytes at 56,
+        // 0 to 4 at 64), and more warps serve them better (4096 worlds: 5.19 against 5.21 ms).
         PersistentTuning shape = tile_tuning;
         if (!tile_tuning_set && per_world > TILE_MAX_INSTANCES) shape.registers = 64;
         // A capture waits for and marks the event each time it is replayed.

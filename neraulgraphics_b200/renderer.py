@@ -406,8 +406,8 @@ class BatchRenderer:
 
     @property
     def last_stage_ms(self) -> list:
-        """The last render's GPU ms by kernel: [camera rays, shading, shadow rays] for the tile kernels, else
-        [whole launch]."""
+        """The last render's GPU ms by kernel: [camera rays, shading, shadow rays] for the tile kernels in one pass, else
+        [whole render]."""
         ms = (C.c_float * 4)()
         n = C.c_int32(0)
         check(self._lib.ngb_last_stage_ms(self._h, ms, 4, C.byref(n)), self._h)

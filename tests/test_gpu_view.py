@@ -7,7 +7,7 @@ The picture of frame k > 0 averages its samples with the frames before it, so a 
 are within one level (CUDA's sinf, cosf and powf against the host's) and depth, normals and IDs bit-exact. The
 scenes cover every kernel the view render runs: the per-pixel kernel (a mirror sphere, two lights, two samples
 per frame), the tile kernels (eight icospheres, one soft-shadow light) and, for the world of 100,000 instances,
-the warp-packet walk with the shadow rays as persistent-kernel jobs.
+the warp-packet walk.
 """
 
 import numpy as np
