@@ -315,10 +315,9 @@ int ngb_set_sync(ngb_renderer *r, int32_t synchronous, double timeout_seconds);
  * candidate lists, larger ones walking their tree as a warp packet), in one pass for one sample per pixel, at most one
  * light and no material with reflectivity >= 1e-3, else a pass per sample and light; the per-pixel kernel where the
  * passes' scratch (77 bytes per pixel, kept) cannot be had: no memory (not tried again for as many pixels until
- * ngb_set_rows), or a stream capture before any such render of the whole image; and, with kernel 0, for images of fewer
- * than 64 + 3/4 P pixels (512 + 3/5 P in worlds of P > 256 instances) that are fewer than 32768 in all, which passes
- * draw slower. 1: the per-pixel kernel.
- * 2: the persistent kernel where it applies (what takes one pass), else the per-pixel kernel.
+ * ngb_set_rows), or a stream capture before any such render of the whole image; and for images of fewer than 64 + 3/4 P
+ * pixels (512 + 3/5 P in worlds of P > 256 instances) that are fewer than 32768 in all, which passes draw slower.
+ * 1: the per-pixel kernel. 2: the persistent kernel where it applies (what takes one pass), else the per-pixel kernel.
  * Ray queries (ngb_cast_rays), unless ngb_set_ray_kernel chose otherwise, take warp packets (kernel 0 or 3; in more than
  * 32768 worlds of at most 256 instances with up to one ray, and at most 16, per 8192 worlds the persistent kernel), the
  * persistent kernel in its shape (kernel 2), or the per-thread ray kernel (kernel 1).

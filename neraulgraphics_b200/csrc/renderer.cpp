@@ -1145,7 +1145,7 @@ void Renderer::render(const float *cams, float fov, int spp, unsigned outputs, i
     }
     // The per-pixel kernel needs no scratch: pictures that the tile kernels take several passes for go to it where the
     // passes' scratch cannot be had.
-    if (tiles && !persistent_ok) tiles = !(kernel_choice == 0 && coarse()) && pass_scratch(a, views, single);
+    if (tiles && !persistent_ok) tiles = !coarse() && pass_scratch(a, views, single);
     const bool in_passes = tiles && !persistent_ok;
     const bool persistent = !view && !tiles && persistent_ok && (kernel_choice == 0 || kernel_choice == 2);
     require(!uneven || tiles, "worlds of uneven sizes render with one sample per pixel, at most one light and no "
